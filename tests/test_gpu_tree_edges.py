@@ -1,0 +1,37 @@
+"""Trees, openings and FRI tails at the edges of their kernels' shapes.
+
+The reduce launch hashes a level of 128 nodes by threads and smaller ones by
+quads of lanes, in stages of 8 levels over blocks of 256; deeper trees start
+with leaf subtrees and node kernels down to 2^16 hashes.  Openings take eight
+lanes per (query, stored-level group), four pairs per warp, and the line folds
+of at most 256 values run in one block."""
+import numpy as np
+import pytest
+
+from gpu_util import to_dev
+from vortexstark_b200 import prover, tune
+from vortexstark_b200.merkle import FusedRoot
+from vortexstark_b200.workload import m31_array
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ncols", [1, 4, 5])
+@pytest.mark.parametrize("log_n", list(range(1, 20)) + [21])
+def test_roots_at_every_depth(oracle, log_n, ncols):
+    cols = [m31_array(31 * log_n + i, 1 << log_n) for i in range(ncols)]
+    want = tuple(oracle.merkle_root(cols).tolist())
+    d = [to_dev(c) for c in cols]
+    for k in (1, 2, 3, 4) if log_n > 16 else (0,):
+        tune.set_leaf_k(log_n, k)
+        try:
+            assert FusedRoot(log_n).commit(d) == want, k
+        finally:
+            tune.set_leaf_k(log_n, 0)
+
+
+@pytest.mark.parametrize("log_n,blowup,nq", [(4, 1, 1), (4, 1, 3), (4, 3, 17), (5, 2, 4), (6, 3, 5), (7, 2, 33),
+                                             (8, 1, 2), (9, 1, 31), (10, 2, 79), (11, 3, 1), (13, 1, 7), (15, 3, 81)])
+def test_proofs_at_odd_query_counts(oracle, log_n, blowup, nq):
+    a, b = 1000 + log_n, 77 * nq
+    assert prover.prove_bytes(a, b, log_n, blowup, nq) == oracle.prove(a, b, log_n, blowup, nq)

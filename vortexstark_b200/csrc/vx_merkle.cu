@@ -42,8 +42,12 @@ uint32_t tree_leaf_k(uint32_t depth, uint32_t kind) {
     // thread, so more threads keep their loads in flight (measured on a
     // 2^26-point FRI chain: 6.08 ms against 6.82 ms with 16 per thread).
     if (kind == kLeafFold) return 2u;
-    // narrow leaves: 2^k leaves per thread, k = 1..4, at least 2^16 threads
-    int k = (int)depth - 17;
+    // narrow leaves: 2^k leaves per thread, k = 1..4, at least 2^18 threads
+    // (7 warps per SM sub-partition) before a thread takes more: the last
+    // wave of few long-running blocks costs more than the larger stored level
+    // (2^20 leaves: 108 us with 4 per thread, 118 us with 8; 2^21: 185 us
+    // with 8, 205 us with 16; 2^22 and deeper: 16 is as good or better)
+    int k = (int)depth - 18;
     return (uint32_t)(k < 1 ? 1 : (k > 4 ? 4 : k));
 }
 
@@ -63,7 +67,11 @@ uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf
     if (depth > 16) {
         h = (leaf_k >= 1 && leaf_k <= 4) ? leaf_k : tree_leaf_k(depth);  // leaf kernel: 2^h leaves per thread
         add(h);
-        while (depth - h > 20) { h += 4; add(h); }  // node kernels, 16 -> 1
+        // node kernels, at most 16 -> 1, down to 2^16 hashes.  A thread of a
+        // node kernel keeps every lane busy; the reduce launch, with a block
+        // of 256 threads per 256 hashes and half of them idle a level later,
+        // takes over where its chain of levels, not the hashing, sets the time.
+        while (depth - h > kReduceLog) { h += depth - h - kReduceLog < 4 ? depth - h - kReduceLog : 4; add(h); }
         lv->top = lv->n - 1;
     }
     // reduce stages of 8 levels from h: every 4th height is stored, so the

@@ -21,6 +21,7 @@
 #include "vx_blake2s.cuh"
 #include "vx_common.cuh"
 #include "vx_field.cuh"
+#include "vx_quad.cuh"
 
 namespace vx {
 
@@ -312,16 +313,48 @@ struct ChanStep {
     uint32_t *proof_root; // 8 words in the proof
     uint32_t *alpha_out;  // null: no draw
 };
-__device__ __forceinline__ void chan_commit(const ChanStep &c, const uint32_t root[8]) {
-    uint32_t m[16];
-#pragma unroll
-    for (int i = 0; i < 8; i++) { m[i] = c.ch->state[i]; m[8 + i] = root[i]; c.proof_root[i] = root[i]; }
-    uint32_t h[8];
-    blake2s_block(h, m, 64u);
-#pragma unroll
-    for (int i = 0; i < 8; i++) c.ch->state[i] = h[i];
-    c.ch->n_draws = 0;
-    if (c.alpha_out) chan_draw_felt(c.ch, c.alpha_out);
+// By one warp whose lane l < 4 holds root[l] (r0) and root[4 + l] (r1) and
+// the channel state's words (s0, s1, updated); msg: 16 shared words.  Every
+// quad of the warp hashes the same message; quad 0 writes.  draw_felt is the
+// same bounded rejection loop as chan_draw_felt; lane l < 4 returns word l of
+// the challenge.
+__device__ __forceinline__ uint32_t chan_commit_quad(const Quad &q, const ChanStep &c, uint32_t *msg, uint32_t &s0,
+                                                     uint32_t &s1, uint32_t r0, uint32_t r1) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane < 4) {
+        msg[lane] = s0; msg[4 + lane] = s1; msg[8 + lane] = r0; msg[12 + lane] = r1;
+        c.proof_root[lane] = r0; c.proof_root[4 + lane] = r1;
+    }
+    uint32_t draws = 0, nbytes = 64u, w0 = 0, w1 = 0;
+    bool ok = true;
+    // pass 0 mixes the root; passes 1.. squeeze with n_draws = pass - 1
+#pragma unroll 1
+    for (uint32_t pass = 0;; pass++) {
+        __syncwarp();
+        quad_hash(q, msg, nbytes, w0, w1);
+        __syncwarp();
+        if (pass == 0) {
+            s0 = w0; s1 = w1;
+            if (lane < 4) {
+                c.ch->state[lane] = w0; c.ch->state[4 + lane] = w1;
+                msg[lane] = w0; msg[4 + lane] = w1; msg[8 + lane] = 0u; msg[12 + lane] = 0u;
+            }
+            if (!c.alpha_out) break;
+            nbytes = 37u;
+            continue;
+        }
+        draws = pass;
+        ok = __all_sync(0xFFFFFFFFu, w0 < 2u * VX_P && w1 < 2u * VX_P);
+        if (ok || pass == 64u) break;
+        if (lane == 0) msg[8] = pass;
+    }
+    w0 = !ok ? 0u : w0 >= VX_P ? w0 - VX_P : w0;
+    if (lane < 4 && c.alpha_out) c.alpha_out[lane] = w0;
+    if (lane == 0) {
+        c.ch->n_draws = draws;
+        if (!ok) c.ch->err = 1u;
+    }
+    return w0;
 }
 
 // Stored levels of one tree: level[0] is the leaf data (via its source),
@@ -331,8 +364,8 @@ __device__ __forceinline__ void chan_commit(const ChanStep &c, const uint32_t ro
 //
 // Build: trees of depth <= 16 go to one multi-block reduce launch straight
 // from the leaves.  Deeper trees: one thread per 2^k-leaf subtree (k = 1..4,
-// chosen so that at least 2^16 threads run), then 16 -> 1 node kernels while
-// a level has more than 2^20 hashes, then the reduce launch for the rest.
+// chosen so that at least 2^16 threads run), then node kernels of at most
+// 16 -> 1 down to 2^16 hashes, then the reduce launch for the rest.
 // The reduce kernel works in stages of up to 8 levels: each block reduces 256
 // hashes in shared memory, one compression per thread per level; the last
 // block of every group of 256 (found with a counter, no waiting) carries on
@@ -348,7 +381,8 @@ struct TreeLevels {
 };
 
 constexpr uint32_t kStageLog = 8;        // levels per reduce stage (256 hashes per block)
-constexpr uint32_t kReduceThreads = 128;
+constexpr uint32_t kReduceThreads = 256;
+constexpr uint32_t kReduceLog = 16;      // the reduce launch starts from at most 2^16 hashes
 
 // Carve the stored levels and counters of a 2^depth-leaf tree from `pool`
 // (null: size only); returns the words used.  Trees deeper than 16 start
@@ -369,77 +403,124 @@ void tree_knob_set(int dev, uint32_t depth, uint32_t k, uint32_t kind = kLeafNar
 // Zero the group counters of a freshly carved tree.
 cudaError_t tree_reset(const TreeLevels &lv, cudaStream_t stream);
 
-// Write this block's part of level `h` if it is a stored level: cnt hashes
-// held at sh, chunk index `part` of that level.
-__device__ __forceinline__ void store_level_part(const TreeLevels &lv, uint32_t h, const uint32_t *sh, uint32_t cnt,
-                                                 uint64_t part) {
-    for (uint32_t i = 1; i < lv.n; i++) {
-        if (lv.height[i] != h) continue;
-        uint4 *dst = (uint4 *)(lv.hashes[i] + 8ull * part * cnt);
-        const uint4 *s4 = (const uint4 *)sh;
-        for (uint32_t j = threadIdx.x; j < 2u * cnt; j += blockDim.x) dst[j] = s4[j];
+// Where node `j` of the level at height h goes if that level is stored (the
+// levels above `top` are stored at every 4th height and at the root).  Height
+// lv.height[top] itself (u = 0) is the level being read, never written here.
+__device__ __forceinline__ uint32_t *stored_node(const TreeLevels &lv, uint32_t h, uint64_t j) {
+    const uint32_t u = h - lv.height[lv.top];
+    if (u == 0u || ((u & 3u) && h != lv.height[lv.n - 1])) return nullptr;
+    return lv.hashes[lv.top + ((u + 3u) >> 2)] + 8ull * j;
+}
+
+// A reduce block holds up to 256 hashes of one level as 128 messages of two
+// children, 20 words apart (16-byte aligned, and consecutive messages start
+// 20 banks apart).  The level of 128 nodes takes one thread per node; from 64
+// nodes down a node is hashed by four lanes (quad_hash), which is what bounds
+// these levels: each is one dependent compression, 650 ns by a quad against
+// 880 ns by a thread.  The last four levels and the transcript step stay in
+// warp 0 without block barriers.
+constexpr uint32_t kMsgWords = 20;
+
+// Levels of `half` <= 64 nodes down to one, from the messages in cur; the
+// first level hashes nbytes of each message, the others 64.  lev: the height
+// of the first level's nodes, part: this block's chunk.  Returns the buffer
+// that no warp reads any more; lanes 0..3 of warp 0 get the last node's words.
+// All threads of the block call it.
+__device__ __forceinline__ uint32_t *quad_levels(const Quad &q, const TreeLevels &lv, uint32_t *cur, uint32_t *nxt,
+                                                 uint32_t half, uint32_t lev, uint64_t part, uint32_t nbytes,
+                                                 uint32_t &o0, uint32_t &o1) {
+    const uint32_t warp = threadIdx.x >> 5, node = threadIdx.x >> 2;
+    o0 = o1 = 0;
+#pragma unroll 1
+    for (; half; half >>= 1, lev++) {
+        if (8u * warp < half) {  // 8 nodes per warp; lanes past the last node hash unused words
+            quad_hash(q, cur + kMsgWords * node, nbytes, o0, o1);
+            if (node < half) {
+                uint32_t *d = nxt + kMsgWords * (node >> 1) + 8u * (node & 1u) + q.l;
+                d[0] = o0; d[4] = o1;
+                uint32_t *g = stored_node(lv, lev, part * half + node);
+                if (g) { g[q.l] = o0; g[4u + q.l] = o1; }
+            }
+        }
+        if (half > 8u) __syncthreads();
+        else __syncwarp();
+        uint32_t *t = cur; cur = nxt; nxt = t;
+        nbytes = 64u;
     }
+    return nxt;
 }
 
 template <class Src>
 __global__ void __launch_bounds__(kReduceThreads) tree_reduce_kernel(Src src, TreeLevels lv, ChanStep cs, uint32_t one) {
-    __shared__ __align__(16) uint32_t sh[8u << kStageLog];
+    __shared__ __align__(16) uint32_t buf[2][128 * kMsgWords];
     __shared__ uint32_t is_last;
+    Quad q;
+    q.init();
     pdl_wait();
     if constexpr (plain_adds<Src>::value) one = 1u;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t depth = lv.height[lv.n - 1];
     uint32_t h = lv.height[lv.top];
     const uint32_t *in = lv.top ? lv.hashes[lv.top] : nullptr;
     uint64_t part = blockIdx.x;     // this block's chunk of the current stage
     uint64_t chunks = gridDim.x;    // chunks of the current stage
     uint32_t cbase = 0;             // first counter of the current stage
+    uint32_t s0 = 0, s1 = 0;        // channel state words of lanes 0..3 of warp 0
+    if (cs.ch && tid < 4) { s0 = __ldcg(cs.ch->state + tid); s1 = __ldcg(cs.ch->state + 4 + tid); }
     while (true) {
         const uint32_t c = depth - h < kStageLog ? depth - h : kStageLog;
         const uint32_t m = 1u << c;
-        if (!in) {
-            src.init();
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                uint32_t hv[8];
-                leaf_digest(src, (part << c) + i, hv, one);
-                store_hash(sh + 8 * i, hv);
+        uint32_t *cur = buf[0], *nxt = buf[1];
+        if (tid < m) {
+            uint32_t hv[8];
+            if (!in) {
+                src.init();
+                leaf_digest(src, (part << c) + tid, hv, one);
+            } else {
+                const uint4 *p = (const uint4 *)(in + 8ull * ((part << c) + tid));
+                const uint4 x = __ldcg(p), y = __ldcg(p + 1);
+                hv[0] = x.x; hv[1] = x.y; hv[2] = x.z; hv[3] = x.w; hv[4] = y.x; hv[5] = y.y; hv[6] = y.z; hv[7] = y.w;
             }
-        } else {
-            const uint4 *p = (const uint4 *)(in + 8ull * (part << c));
-            for (uint32_t j = threadIdx.x; j < 2u * m; j += blockDim.x) ((uint4 *)sh)[j] = __ldcg(p + j);
+            store_hash(cur + kMsgWords * (tid >> 1) + 8u * (tid & 1u), hv);
         }
         __syncthreads();
-        for (uint32_t d = 0; d < c; d++) {
-            const uint32_t half = m >> (d + 1);
-            for (uint32_t base = 0; base < half; base += blockDim.x) {
-                const uint32_t t = base + threadIdx.x;
+        uint32_t half = m >> 1, lev = h + 1;
+        if (half == 128u) {
+            if (tid < 128u) {
                 uint32_t hv[8];
-                const bool act = t < half;
-                if (act) blake2s_node(hv, sh + 16 * t, sh + 16 * t + 8, one);
-                __syncthreads();
-                if (act) store_hash(sh + 8 * t, hv);
-                __syncthreads();
+                blake2s_node(hv, cur + kMsgWords * tid, cur + kMsgWords * tid + 8, one);
+                store_hash(nxt + kMsgWords * (tid >> 1) + 8u * (tid & 1u), hv);
+                uint32_t *g = stored_node(lv, lev, part * 128u + tid);
+                if (g) store_hash(g, hv);
             }
-            store_level_part(lv, h + d + 1, sh, half, part);
+            __syncthreads();
+            uint32_t *t = cur; cur = nxt; nxt = t;
+            half = 64u; lev++;
         }
+        uint32_t o0, o1;
+        nxt = quad_levels(q, lv, cur, nxt, half, lev, part, 64u, o0, o1);
         h += c;
         if (h == depth) {
-            if (threadIdx.x == 0 && cs.ch) chan_commit(cs, sh);
+            if (cs.ch && warp == 0) chan_commit_quad(q, cs, nxt, s0, s1, o0, o1);
             return;
         }
-        // this chunk's root is in the stored level at height h; the last
-        // block of each group of 2^cn chunks reduces the group next
+        // this chunk's root is in the stored level at height h (written by
+        // lanes 0..3); the last block of each group of 2^cn chunks reduces the
+        // group next
         const uint32_t cn = depth - h < kStageLog ? depth - h : kStageLog;
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t *ctr = lv.cnt + cbase + (part >> cn);
-            uint32_t old = atomicAdd(ctr, 1u);
-            is_last = old == (1u << cn) - 1u;
-            if (is_last) *ctr = 0u;  // every block of the group has arrived: ready for the next launch
+        if (warp == 0) {
+            __threadfence();
+            __syncwarp();
+            if (tid == 0) {
+                uint32_t *ctr = lv.cnt + cbase + (part >> cn);
+                uint32_t old = atomicAdd(ctr, 1u);
+                is_last = old == (1u << cn) - 1u;
+                if (is_last) *ctr = 0u;  // every block of the group has arrived: ready for the next launch
+                __threadfence();
+            }
         }
         __syncthreads();
         if (!is_last) return;
-        __threadfence();
         cbase += (uint32_t)(chunks >> cn);
         chunks >>= cn;
         part >>= cn;
