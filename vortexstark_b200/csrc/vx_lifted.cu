@@ -28,6 +28,7 @@
 #include "vx_fri.cuh"
 #include "vx_merkle.cuh"
 #include "vx_ntt.cuh"
+#include "vx_paths.cuh"
 #include "vx_prover.cuh"
 #include "vx_twiddles.cuh"
 
@@ -250,23 +251,20 @@ __global__ void lift_queries_kernel(DevChannel *ch, const uint32_t *l0, const ui
 
 // Opened values: thread (tree, q); tree 0 = lifted rows, 1 = C, 2 + k = FRI layer k.
 struct LiftValuesArgs {
-    LeafLifted cols;
     const uint32_t *C[4];
     const uint32_t *F[kMaxFri][4];
     uint64_t vals[2 + kMaxFri], svals[2 + kMaxFri];
     uint32_t nfri;
 };
-__global__ void lift_values_kernel(const __grid_constant__ LiftValuesArgs a, const uint32_t *qidx, uint32_t nq,
-                                   uint32_t *proof) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= (2 + a.nfri) * nq) return;
-    const uint32_t tree = tid / nq, q = tid % nq;
+__device__ __forceinline__ void lift_value(const LiftValuesArgs &a, const LeafLifted &cols, uint32_t item, const uint32_t *qidx, uint32_t nq,
+                                           uint32_t *proof) {
+    const uint32_t tree = item / nq, q = item % nq;
     const uint64_t i = qidx[q];
     if (tree == 0) {
-        const uint32_t nc = a.cols.n_cols;
+        const uint32_t nc = cols.n_cols;
         for (uint32_t c = 0; c < nc; c++) {
-            proof[a.vals[0] + (uint64_t)q * nc + c] = a.cols.word(c, i);
-            proof[a.svals[0] + (uint64_t)q * nc + c] = a.cols.word(c, i ^ 1ull);
+            proof[a.vals[0] + (uint64_t)q * nc + c] = cols.word(c, i);
+            proof[a.svals[0] + (uint64_t)q * nc + c] = cols.word(c, i ^ 1ull);
         }
     } else if (tree == 1) {
         for (int c = 0; c < 4; c++) {
@@ -283,9 +281,9 @@ __global__ void lift_values_kernel(const __grid_constant__ LiftValuesArgs a, con
     }
 }
 
-// Authentication paths: blockIdx.y = tree, threads over (query, stored-level
-// group); each rebuilds the <= 16-leaf block of its group from the level
-// below (or the leaves) and writes the siblings of its heights.
+// All openings in one launch: blockIdx.y = tree, eight lanes per (stored-level
+// group, query) pair of its authentication paths; the blocks past the last
+// tree write the opened values.
 struct LiftPathTree {
     TreeLevels lv;
     uint32_t kind;   // 0 lifted rows, 1 SoA4 columns
@@ -297,61 +295,36 @@ struct LiftPathsArgs {
     LeafLifted cols;
     LiftPathTree t[2 + kMaxFri];
 };
-__global__ void __launch_bounds__(64) lift_paths_kernel(const __grid_constant__ LiftPathsArgs a, const uint32_t *qidx,
-                                                        uint32_t nq, uint32_t *proof) {
+__global__ void __launch_bounds__(kPathThreads) lift_paths_kernel(const __grid_constant__ LiftPathsArgs a,
+                                                                  const __grid_constant__ LiftValuesArgs va,
+                                                                  const uint32_t *qidx, uint32_t nq, uint32_t *proof) {
+    __shared__ __align__(16) uint32_t nh[kPathItems * kPathWords];
+    pdl_wait();
+    const uint32_t ntree = 2 + va.nfri;
+    if (blockIdx.y == ntree) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ntree * nq; i += gridDim.x * blockDim.x)
+            lift_value(va, a.cols, i, qidx, nq, proof);
+        return;
+    }
     const LiftPathTree &T = a.t[blockIdx.y];
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t ng = T.lv.n - 1;
-    if (tid >= nq * ng) return;
-    const uint32_t q = tid / ng, g = tid % ng;
+    const uint32_t ng = T.lv.n - 1, slot = threadIdx.x / kPathLanes, item = blockIdx.x * kPathItems + slot;
+    const bool act = item < nq * ng;
+    const uint32_t g = act ? item / nq : 0u, q = act ? item % nq : 0u;  // a warp's pairs share their group
     const uint32_t depth = T.lv.height[T.lv.n - 1];
     const uint64_t idx = (uint64_t)qidx[q] >> T.shift;
-    const uint32_t lo = T.lv.height[g], k = T.lv.height[g + 1] - lo;
-    const uint64_t node = idx >> lo;
-    const uint64_t blk = node >> k;
-    const uint32_t K = 1u << k;
-    uint32_t nh[31][8];
-    if (g == 0) {
-        for (uint32_t j = 0; j < K; j++) {
-            const uint64_t i = (blk << k) + j;
-            if (T.kind == 0) {
-                a.cols.digest(i, nh[j]);
-            } else {
-                uint32_t m[16];
+    auto leaf = [&](uint64_t i, uint32_t h[8]) {
+        if (T.kind == 0) {
+            a.cols.digest(i, h);
+        } else {
+            uint32_t m[16];
 #pragma unroll
-                for (int w = 0; w < 16; w++) m[w] = 0u;
-                m[0] = T.c[0][i]; m[1] = T.c[1][i]; m[2] = T.c[2][i]; m[3] = T.c[3][i];
-                blake2s_block(nh[j], m, 16u);
-            }
+            for (int w = 0; w < 16; w++) m[w] = 0u;
+            m[0] = T.c[0][i]; m[1] = T.c[1][i]; m[2] = T.c[2][i]; m[3] = T.c[3][i];
+            blake2s_block(h, m, 16u);
         }
-    } else {
-        const uint32_t *h = T.lv.hashes[g] + 8ull * (blk << k);
-        for (uint32_t j = 0; j < K; j++)
-#pragma unroll
-            for (int w = 0; w < 8; w++) nh[j][w] = h[8 * j + w];
-    }
-    uint32_t off = 0, cnt = K;
-    for (uint32_t d = 0; d < k; d++) {
-        const uint32_t nxt = off + cnt;
-        for (uint32_t j = 0; j < cnt / 2; j++) blake2s_node(nh[nxt + j], nh[off + 2 * j], nh[off + 2 * j + 1]);
-        off = nxt;
-        cnt /= 2;
-    }
-    uint32_t *p = proof + T.paths + (uint64_t)q * (1u + 8u * depth);
-    uint32_t *sp = proof + T.spaths + (uint64_t)q * (1u + 8u * depth);
-    off = 0; cnt = K;
-    uint64_t local = node & (K - 1u);
-    for (uint32_t d = 0; d < k; d++) {
-        const uint32_t hgt = lo + d;
-        const uint32_t *sib = nh[off + (uint32_t)(local ^ 1u)];
-        const uint32_t *self = nh[off + (uint32_t)local];
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            p[1 + 8 * hgt + w] = sib[w];
-            sp[1 + 8 * hgt + w] = (hgt == 0) ? self[w] : sib[w];
-        }
-        off += cnt; cnt /= 2; local >>= 1;
-    }
+    };
+    path_group(leaf, T.lv, g, idx, act, nh + kPathWords * slot, proof + T.paths + (uint64_t)q * (1u + 8u * depth),
+               proof + T.spaths + (uint64_t)q * (1u + 8u * depth));
 }
 
 uint64_t align64(uint64_t w) { return (w + 63) & ~63ull; }
@@ -499,7 +472,6 @@ int lift_stage(vx_lifted *h, uint32_t stage, cudaStream_t st, uint32_t *launches
     case 6: {
         LiftValuesArgs va;
         memset(&va, 0, sizeof(va));
-        va.cols = h->cols;
         va.nfri = L.nfri;
         for (int c = 0; c < 4; c++) va.C[c] = h->C[c];
         va.vals[0] = L.lift.vals; va.svals[0] = L.lift.svals;
@@ -508,7 +480,6 @@ int lift_stage(vx_lifted *h, uint32_t stage, cudaStream_t st, uint32_t *launches
             for (int c = 0; c < 4; c++) va.F[k][c] = h->F[k][c];
             va.vals[2 + k] = L.fri[k].vals; va.svals[2 + k] = L.fri[k].svals;
         }
-        lift_values_kernel<<<blocks_for((uint64_t)(2 + L.nfri) * L.nq, 128), 128, 0, st>>>(va, h->qidx, L.nq, proof);
         LiftPathsArgs pa;
         memset(&pa, 0, sizeof(pa));
         pa.cols = h->cols;
@@ -523,9 +494,10 @@ int lift_stage(vx_lifted *h, uint32_t stage, cudaStream_t st, uint32_t *launches
         add(0, h->lv0, 0, 0, nullptr, L.lift);
         add(1, h->lv1, 1, 0, h->C, L.comb);
         for (uint32_t k = 0; k < L.nfri; k++) add(2 + k, h->flv[k], 1, k + 1, h->F[k], L.fri[k]);
-        dim3 grid(blocks_for((uint64_t)L.nq * max_groups, 64), 2 + L.nfri);
-        lift_paths_kernel<<<grid, 64, 0, st>>>(pa, h->qidx, L.nq, proof);
-        *launches += 2;
+        dim3 grid(blocks_for((uint64_t)L.nq * max_groups, kPathItems), 3 + L.nfri);
+        VX_CUDA_TRY(launch_pdl(lift_paths_kernel, grid, dim3(kPathThreads), 0, st, pa, va, (const uint32_t *)h->qidx,
+                               L.nq, proof));
+        *launches += 1;
         break;
     }
     default:

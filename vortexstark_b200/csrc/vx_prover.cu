@@ -21,6 +21,7 @@
 #include "vx_fri.cuh"
 #include "vx_merkle.cuh"
 #include "vx_ntt.cuh"
+#include "vx_paths.cuh"
 #include "vx_prover.cuh"
 #include "vx_twiddles.cuh"
 
@@ -128,14 +129,17 @@ __device__ __forceinline__ void fib_step(uint32_t &g0, uint32_t &g1, const uint3
 // (G(base), G(base + 1)) from the powers-of-two table, every thread derives
 // its 32-row chunk's seed with one table step, runs the recurrence into
 // shared memory, and the block writes its rows coalesced.  Also stamps
-// (a, b) into the proof header.
+// (a, b) into the proof header and starts the transcript.
 constexpr uint32_t kTraceRows = 8192;
 __global__ void __launch_bounds__(256) fib_trace_kernel(uint32_t a, uint32_t b, const uint32_t *ab_dev, uint32_t *out,
-                                                        uint64_t n, uint32_t *proof_ab) {
+                                                        uint64_t n, uint32_t *proof_ab, DevChannel *ch) {
     __shared__ uint32_t rows[256 * 33];
     __shared__ uint32_t seed[2];
     if (ab_dev) { a = ab_dev[0]; b = ab_dev[1]; }
-    if (blockIdx.x == 0 && threadIdx.x == 0) { proof_ab[0] = a; proof_ab[1] = b; }
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) { proof_ab[0] = a; proof_ab[1] = b; }
+        if (threadIdx.x < sizeof(DevChannel) / 4) ((uint32_t *)ch)[threadIdx.x] = 0u;
+    }
     const uint64_t base = (uint64_t)blockIdx.x * kTraceRows;
     if (threadIdx.x == 0) {
         uint32_t g0 = a, g1 = b;
@@ -240,11 +244,9 @@ struct ValuesArgs {
     uint64_t vals[34], svals[34];
     uint32_t nfri;
 };
-__global__ void decommit_values_kernel(ValuesArgs a, const uint32_t *qidx, uint32_t nq, uint32_t *proof) {
-    uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t ntree = 2 + a.nfri;
-    if (tid >= ntree * nq) return;
-    uint32_t tree = tid / nq, q = tid % nq;
+__device__ __forceinline__ void decommit_value(const ValuesArgs &a, uint32_t item, const uint32_t *qidx, uint32_t nq,
+                                               uint32_t *proof) {
+    uint32_t tree = item / nq, q = item % nq;
     uint64_t i = qidx[q];
     if (tree == 0) {
         proof[a.vals[0] + q] = a.eval[i];
@@ -264,9 +266,10 @@ __global__ void decommit_values_kernel(ValuesArgs a, const uint32_t *qidx, uint3
     }
 }
 
-// All authentication paths of a proof in one launch: blockIdx.y selects the
-// tree (0 trace, 1 quotient, 2 + k FRI layer k), threads cover
-// (query, stored-level group) pairs of that tree.
+// All openings of a proof in one launch: blockIdx.y selects the tree (0 trace,
+// 1 quotient, 2 + k FRI layer k) whose authentication paths the block's
+// groups of eight lanes rebuild, one (stored-level group, query) pair each;
+// the blocks past the last tree write the opened values.
 struct PathTree {
     TreeLevels lv;
     uint32_t kind;    // 0: M31 eval column, 1: quotient from eval, 2: SoA4 layer
@@ -280,62 +283,38 @@ struct PathsArgs {
     uint64_t mask;
     const uint32_t *alpha_q;
 };
-__global__ void __launch_bounds__(64) decommit_all_kernel(const __grid_constant__ PathsArgs a, const uint32_t *qidx,
-                                                          uint32_t nq, uint32_t *proof) {
+__global__ void __launch_bounds__(kPathThreads) decommit_all_kernel(const __grid_constant__ PathsArgs a,
+                                                                    const __grid_constant__ ValuesArgs va,
+                                                                    const uint32_t *qidx, uint32_t nq,
+                                                                    uint32_t *proof) {
+    __shared__ __align__(16) uint32_t nh[kPathItems * kPathWords];
+    pdl_wait();
+    const uint32_t ntree = 2 + va.nfri;
+    if (blockIdx.y == ntree) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ntree * nq; i += gridDim.x * blockDim.x)
+            decommit_value(va, i, qidx, nq, proof);
+        return;
+    }
     const PathTree &T = a.t[blockIdx.y];
-    uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t ng = T.lv.n - 1;
-    if (tid >= nq * ng) return;
-    uint32_t q = tid / ng, g = tid % ng;
-    uint32_t depth = T.lv.height[T.lv.n - 1];
-    uint64_t idx = (uint64_t)qidx[q] >> T.shift;
-    uint32_t lo = T.lv.height[g], k = T.lv.height[g + 1] - lo;
-    uint64_t node = idx >> lo;
-    uint64_t blk = node >> k;
-    const uint32_t K = 1u << k;
-    uint32_t nh[31][8];
-    if (g == 0) {
-        LeafQuotient lq{a.eval, a.mask, a.alpha_q, {0, 0, 0, 0}};
-        if (T.kind == 1) lq.init();
-        for (uint32_t j = 0; j < K; j++) {
-            uint32_t m[16];
+    const uint32_t ng = T.lv.n - 1, slot = threadIdx.x / kPathLanes, item = blockIdx.x * kPathItems + slot;
+    const bool act = item < nq * ng;
+    const uint32_t g = act ? item / nq : 0u, q = act ? item % nq : 0u;  // a warp's pairs share their group
+    const uint32_t depth = T.lv.height[T.lv.n - 1];
+    const uint64_t idx = (uint64_t)qidx[q] >> T.shift;
+    LeafQuotient lq{a.eval, a.mask, a.alpha_q, {0, 0, 0, 0}};
+    if (T.kind == 1) lq.init();
+    auto leaf = [&](uint64_t i, uint32_t h[8]) {
+        uint32_t m[16];
 #pragma unroll
-            for (int w = 0; w < 16; w++) m[w] = 0u;
-            uint64_t i = (blk << k) + j;
-            uint32_t nb;
-            if (T.kind == 0) { m[0] = T.c[0][i]; nb = 4u; }
-            else if (T.kind == 1) { nb = lq.load(i, m); }
-            else { m[0] = T.c[0][i]; m[1] = T.c[1][i]; m[2] = T.c[2][i]; m[3] = T.c[3][i]; nb = 16u; }
-            blake2s_block(nh[j], m, nb);
-        }
-    } else {
-        const uint32_t *h = T.lv.hashes[g] + 8ull * (blk << k);
-        for (uint32_t j = 0; j < K; j++)
-#pragma unroll
-            for (int w = 0; w < 8; w++) nh[j][w] = h[8 * j + w];
-    }
-    uint32_t lvl_off = 0, cnt = K;
-    for (uint32_t d = 0; d < k; d++) {
-        uint32_t nxt = lvl_off + cnt;
-        for (uint32_t j = 0; j < cnt / 2; j++) blake2s_node(nh[nxt + j], nh[lvl_off + 2 * j], nh[lvl_off + 2 * j + 1]);
-        lvl_off = nxt;
-        cnt /= 2;
-    }
-    uint32_t *p = proof + T.paths + (uint64_t)q * (1u + 8u * depth);
-    uint32_t *sp = proof + T.spaths + (uint64_t)q * (1u + 8u * depth);
-    lvl_off = 0; cnt = K;
-    uint64_t local = node & (K - 1u);
-    for (uint32_t d = 0; d < k; d++) {
-        uint32_t hgt = lo + d;
-        const uint32_t *sib = nh[lvl_off + (uint32_t)(local ^ 1u)];
-        const uint32_t *self = nh[lvl_off + (uint32_t)local];
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            p[1 + 8 * hgt + w] = sib[w];
-            sp[1 + 8 * hgt + w] = (hgt == 0) ? self[w] : sib[w];
-        }
-        lvl_off += cnt; cnt /= 2; local >>= 1;
-    }
+        for (int w = 0; w < 16; w++) m[w] = 0u;
+        uint32_t nb = 16u;
+        if (T.kind == 0) { m[0] = T.c[0][i]; nb = 4u; }
+        else if (T.kind == 1) { lq.load(i, m); }
+        else { m[0] = T.c[0][i]; m[1] = T.c[1][i]; m[2] = T.c[2][i]; m[3] = T.c[3][i]; }
+        blake2s_block(h, m, nb);
+    };
+    path_group(leaf, T.lv, g, idx, act, nh + kPathWords * slot, proof + T.paths + (uint64_t)q * (1u + 8u * depth),
+               proof + T.spaths + (uint64_t)q * (1u + 8u * depth));
 }
 
 }  // namespace
@@ -561,9 +540,8 @@ static int enqueue_stage(vx_prover *p, uint32_t stage, uint32_t a, uint32_t b, c
     auto ntt_launches = [](uint32_t layers, uint32_t elems_log) { return ntt_pass_count(layers, elems_log); };
     switch (stage) {
     case 0:
-        VX_CUDA_TRY(cudaMemsetAsync(S.chan, 0, sizeof(DevChannel), st));
         fib_trace_kernel<<<(unsigned)((n + kTraceRows - 1) / kTraceRows), 256, 0, st>>>(a, b, S.inputs, S.coeffs, n,
-                                                                         proof + L.magic + 3);
+                                                                         proof + L.magic + 3, S.chan);
         *launches += 1;
         break;
     case 1: {
@@ -625,7 +603,6 @@ static int enqueue_stage(vx_prover *p, uint32_t stage, uint32_t a, uint32_t b, c
             for (int c = 0; c < 4; c++) va.fri[k][c] = S.fri[k][c];
             va.vals[2 + k] = L.fri[k].vals; va.svals[2 + k] = L.fri[k].svals;
         }
-        decommit_values_kernel<<<blocks_for((uint64_t)(2 + L.nfri) * L.nq, 128), 128, 0, st>>>(va, S.qidx, L.nq, proof);
         PathsArgs pa;
         memset(&pa, 0, sizeof(pa));
         pa.eval = S.eval; pa.mask = N - 1; pa.alpha_q = S.alpha_q;
@@ -641,9 +618,10 @@ static int enqueue_stage(vx_prover *p, uint32_t stage, uint32_t a, uint32_t b, c
         add(0, S.trace_lv, 0, 0, ev4, L.trace);
         add(1, S.quot_lv, 1, 0, nullptr, L.quot);
         for (uint32_t k = 0; k < L.nfri; k++) add(2 + k, S.fri_lv[k], 2, k + 1, S.fri[k], L.fri[k]);
-        dim3 grid(blocks_for((uint64_t)L.nq * max_groups, 64), 2 + L.nfri);
-        decommit_all_kernel<<<grid, 64, 0, st>>>(pa, S.qidx, L.nq, proof);
-        *launches += 2;
+        dim3 grid(blocks_for((uint64_t)L.nq * max_groups, kPathItems), 3 + L.nfri);
+        VX_CUDA_TRY(launch_pdl(decommit_all_kernel, grid, dim3(kPathThreads), 0, st, pa, va, (const uint32_t *)S.qidx,
+                               L.nq, proof));
+        *launches += 1;
         break;
     }
     default:
