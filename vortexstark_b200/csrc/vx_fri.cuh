@@ -3,6 +3,7 @@
 #include <cstdint>
 
 #include "vx_field.cuh"
+#include "vx_merkle.cuh"
 
 namespace vx {
 
@@ -29,5 +30,63 @@ struct LeafFold {
         return 16u;
     }
 };
+
+// The last FRI layers, of at most 2^kTailLog values each, in one single-block
+// launch: fold, tree and transcript step of every layer, with the folded
+// values, messages and transcript state in shared memory.
+constexpr uint32_t kTailLog = 8;
+struct FriTailLayer {
+    const uint32_t *tw;
+    uint32_t *out[4];
+    uint32_t *root;       // 8 words in the proof
+    uint32_t *alpha_out;  // challenge drawn after this layer; null: none
+    TreeLevels lv;
+};
+struct FriTailArgs {
+    const uint32_t *in[4];     // the layer before, 2^(d0 + 1) values
+    const uint32_t *alpha_in;  // challenge of the first fold
+    DevChannel *ch;
+    uint32_t n, d0;            // layers; log size of the first
+    FriTailLayer l[kTailLog];
+};
+cudaError_t fri_tail(const FriTailArgs &a, cudaStream_t stream);
+
+// Line folds of layers k0 .. k1 - 1: layer k (log size log0 - k, columns
+// F[k][0..3]) folds layer k - 1 with twiddles tw(k) and challenge
+// alpha + 4 k, is committed as tree lv[k], its root goes to root(k), and
+// challenge alpha + 4 (k + 1) is drawn unless k + 1 == n.  Layers of at most
+// 2^kTailLog values share one launch.
+template <class Tw, class Cols, class Root>
+cudaError_t fri_line_layers(uint32_t k0, uint32_t k1, uint32_t n, uint32_t log0, const Cols &F, const TreeLevels *lv,
+                            const Tw &tw, uint32_t *alpha, DevChannel *ch, const Root &root, cudaStream_t st,
+                            uint32_t *launches) {
+    for (uint32_t k = k0; k < k1; k++) {
+        auto next_alpha = [&](uint32_t j) { return j + 1 < n ? alpha + 4 * (j + 1) : nullptr; };
+        if (log0 - k <= kTailLog && k1 - k <= kTailLog) {
+            FriTailArgs a{};
+            for (int c = 0; c < 4; c++) a.in[c] = F(k - 1)[c];
+            a.alpha_in = alpha + 4 * k;
+            a.ch = ch;
+            a.n = k1 - k;
+            a.d0 = log0 - k;
+            for (uint32_t j = k; j < k1; j++) {
+                FriTailLayer &t = a.l[j - k];
+                t.tw = tw(j);
+                for (int c = 0; c < 4; c++) t.out[c] = F(j)[c];
+                t.root = root(j);
+                t.alpha_out = next_alpha(j);
+                t.lv = lv[j];
+            }
+            *launches += 1;
+            return fri_tail(a, st);
+        }
+        uint32_t *const *in = F(k - 1), *const *out = F(k);
+        LeafFold lf{in[0], in[1], in[2], in[3], tw(k), alpha + 4 * k, out[0], out[1], out[2], out[3], {}};
+        cudaError_t e = tree_build(lf, lv[k], ChanStep{ch, root(k), next_alpha(k)}, st);
+        if (e != cudaSuccess) return e;
+        *launches += tree_launches(lv[k]);
+    }
+    return cudaSuccess;
+}
 
 }  // namespace vx

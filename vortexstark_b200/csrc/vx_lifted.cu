@@ -450,17 +450,10 @@ int lift_stage(vx_lifted *h, uint32_t stage, cudaStream_t st, uint32_t *launches
         break;
     }
     case 4:  // line folds
-        for (uint32_t k = 1; k < L.nfri; k++) {
-            const uint32_t lsrc = S - k;
-            LeafFold lf{h->F[k - 1][0], h->F[k - 1][1], h->F[k - 1][2], h->F[k - 1][3],
-                        h->fold_line + h->fold_line_off[lsrc], h->alpha_f + 4 * k,
-                        h->F[k][0], h->F[k][1], h->F[k][2], h->F[k][3], {}};
-            VX_CUDA_TRY(tree_build(lf, h->flv[k],
-                                   ChanStep{h->chan, proof + L.froots + 8 * k,
-                                            k + 1 < L.nfri ? h->alpha_f + 4 * (k + 1) : nullptr},
-                                   st));
-            *launches += tree_launches(h->flv[k]);
-        }
+        VX_CUDA_TRY(fri_line_layers(
+            1, L.nfri, L.nfri, S - 1, [&](uint32_t k) { return h->F[k]; }, h->flv,
+            [&](uint32_t k) { return h->fold_line + h->fold_line_off[S - k]; }, h->alpha_f, h->chan,
+            [&](uint32_t k) { return proof + L.froots + 8 * k; }, st, launches));
         break;
     case 5: {
         const uint32_t kl = L.nfri - 1;

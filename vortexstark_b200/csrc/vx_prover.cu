@@ -574,17 +574,10 @@ static int enqueue_stage(vx_prover *p, uint32_t stage, uint32_t a, uint32_t b, c
         break;
     }
     case 6:
-        for (uint32_t k = k_lo < 1 ? 1 : k_lo; k < L.nfri && k < k_hi; k++) {
-            uint32_t lsrc = le - k;  // log size of the layer being folded
-            LeafLineFold lf{S.fri[k - 1][0], S.fri[k - 1][1], S.fri[k - 1][2], S.fri[k - 1][3],
-                            T.fold_line + T.fold_line_off[lsrc], S.alpha_f + 4 * k,
-                            S.fri[k][0], S.fri[k][1], S.fri[k][2], S.fri[k][3], {}};
-            VX_CUDA_TRY(tree_build(lf, S.fri_lv[k],
-                                   ChanStep{S.chan, proof + L.froots + 8 * k,
-                                            k + 1 < L.nfri ? S.alpha_f + 4 * (k + 1) : nullptr},
-                                   st));
-            *launches += tree_launches(S.fri_lv[k]);
-        }
+        VX_CUDA_TRY(fri_line_layers(
+            k_lo < 1 ? 1 : k_lo, L.nfri < k_hi ? L.nfri : k_hi, L.nfri, le - 1, [&](uint32_t k) { return S.fri[k]; },
+            S.fri_lv, [&](uint32_t k) { return T.fold_line + T.fold_line_off[le - k]; }, S.alpha_f, S.chan,
+            [&](uint32_t k) { return proof + L.froots + 8 * k; }, st, launches));
         break;
     case 7: {
         uint32_t kl = L.nfri - 1;
