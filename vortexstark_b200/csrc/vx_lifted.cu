@@ -207,14 +207,18 @@ struct LeafCombine {
     }
 };
 
-__global__ void powers_kernel(const uint32_t *alpha, uint32_t *pw, uint32_t n) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const qm31 a{{alpha[0], alpha[1], alpha[2], alpha[3]}};
-    qm31 p{{1u, 0u, 0u, 0u}};
-    for (uint32_t c = 0; c < n; c++) {
-        pw[4 * c] = p.v[0]; pw[4 * c + 1] = p.v[1]; pw[4 * c + 2] = p.v[2]; pw[4 * c + 3] = p.v[3];
-        p = qmul(p, a);
+// pw[c] = alpha^c, a thread per power by squaring: 6 dependent steps instead
+// of a chain of n products on one thread.
+__global__ void __launch_bounds__(kMaxLiftCols) powers_kernel(const uint32_t *alpha, uint32_t *pw, uint32_t n) {
+    pdl_wait();
+    const uint32_t c = threadIdx.x;
+    if (c >= n) return;
+    qm31 a{{alpha[0], alpha[1], alpha[2], alpha[3]}}, p{{1u, 0u, 0u, 0u}};
+    for (uint32_t e = c; e; e >>= 1) {
+        if (e & 1u) p = qmul(p, a);
+        a = qmul(a, a);
     }
+    ((uint4 *)pw)[c] = make_uint4(p.v[0], p.v[1], p.v[2], p.v[3]);
 }
 
 // mix_felts(last layer) (channel.rs:46-59), then draw_query_indices: squeeze
@@ -411,7 +415,8 @@ int lift_stage(vx_lifted *h, uint32_t stage, cudaStream_t st, uint32_t *launches
         *launches += tree_launches(h->lv0);
         break;
     case 2: {  // C = sum alpha^c lift(col_c), committed; draw the first fold challenge
-        powers_kernel<<<1, 32, 0, st>>>(h->alpha, h->pw, L.n_cols);
+        VX_CUDA_TRY(launch_pdl(powers_kernel, dim3(1), dim3(kMaxLiftCols), 0, st, (const uint32_t *)h->alpha, h->pw,
+                               L.n_cols));
         CombineGroupsArgs ca;
         memset(&ca, 0, sizeof(ca));
         LeafCombine lc;
