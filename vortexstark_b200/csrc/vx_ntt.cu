@@ -122,6 +122,7 @@ struct Pass2Args {
     uint32_t scale;   // output scale (1 = none)
     uint32_t vec;     // 1: columns and source 16-byte aligned, 4 consecutive elements per access
     uint32_t hb_log;  // > 0: the 2^hb_log tiles that read the same source tile are consecutive blocks
+    uint64_t n_elems; // words per column
 };
 
 // Butterfly products: with a doubled twiddle (mmul_t2: one multiply, one
@@ -367,12 +368,295 @@ __global__ void __launch_bounds__(NT, min_blocks_for(NT)) ntt_tile_kernel(Pass2A
     tile_pass<FWD, R, WL, NT>(p, blockIdx.x, blockIdx.y, dsm);
 }
 
+// Resident blocks per SM the vector pass is compiled for: 8 (64 registers)
+// against 6 or 5: 2^26 evaluate 381 us, 405 and 405; LDE of the 34-column
+// commitment 358 us against 384 with 6.
+#ifndef VX_NTT_VEC_BLOCKS
+#define VX_NTT_VEC_BLOCKS 8
+#endif
+// ---------------------------------------------------------------------
+// Vector pass: a block of 128 threads transforms 4096 elements, 32 per
+// thread, held as 8 groups of 4 consecutive words.  Bound: instruction issue
+// and the integer pipes (a butterfly alone is 7.5 instructions), so the split
+// keeps everything around the butterflies cheap:
+//  - Elements that differ only in their two low index bits share every
+//    twiddle above layer 1, so a twiddle is loaded and doubled once for four
+//    butterflies, and global and shared memory move 16 bytes per access.
+//  - A stage applies up to three layers, those of the index bits of the
+//    thread's 8 groups (bits [A, A+3)); layers 0 and 1 pair words of one
+//    group and need no exchange of their own.
+//  - The first stage takes its elements straight from global memory and the
+//    last one stores them there; only the stages between go through shared
+//    memory (16-byte rows, 4 words of padding per 32).  The stage on bits
+//    [2, 5) holds 32 consecutive words per thread, so its global side is
+//    turned through shared memory, within a warp, to stay coalesced.
+//  - Twiddles come from global memory as aligned runs of 1..16 words per
+//    layer; nothing is staged or decoded per tile.
+// Against 16 elements per thread with the tile and its twiddles staged in
+// shared memory (12.2-15.2 instructions per butterfly): 2^24 evaluate 134 ->
+// 108 us, interpolate 135 -> 120, 2^26 494 -> 381 and 504 -> 436, 16 columns
+// of 2^20 158 -> 101, each through its synchronous launcher.
+// A bottom pass (WL = 0, layers 0 .. R-1, R = 5..12) takes 4096 consecutive
+// elements, 2^(12-R) tiles, per block; an upper pass (R = 3..9, WL = 12 - R)
+// one tile of 2^R rows of 2^WL words.
+// ---------------------------------------------------------------------
+constexpr uint32_t kVecThreads = 128;
+constexpr uint32_t kVecTile = 4096;
+constexpr uint32_t kVecSmemWords = kVecTile + kVecTile / 8;
+__host__ __device__ constexpr uint32_t vpad(uint32_t e) { return e + ((e >> 5) << 2); }
+
+template <bool FWD, int R, int WL, int K>
+struct VecStage {
+    static constexpr int B0 = WL > 2 ? WL : 2;       // lowest index bit of a row layer
+    static constexpr int TB = R + WL;                // index bits of the pass's layers: below TB
+    static constexpr int NST = (TB - B0 + 2) / 3;
+    static constexpr int IDX = FWD ? NST - 1 - K : K;
+    static constexpr int LO = B0 + 3 * IDX;
+    static constexpr int HI = LO + 3 < TB ? LO + 3 : TB;
+    static constexpr int A = LO < TB - 3 ? LO : TB - 3;
+    static constexpr bool TURN = WL == 0 && A == 2;  // 32 consecutive words per thread
+};
+
+// N consecutive words from p (N-aligned index), as wide as `al` allows.
+template <int N>
+__device__ __forceinline__ void load_run(uint32_t t[N], const uint32_t *__restrict__ p, bool al) {
+    if (N == 1 || !al) {
+#pragma unroll
+        for (int i = 0; i < N; i++) t[i] = __ldg(p + i);
+    } else if constexpr (N == 2) {
+        const uint2 x = __ldg((const uint2 *)p);
+        t[0] = x.x; t[1] = x.y;
+    } else if constexpr (N >= 4) {
+#pragma unroll
+        for (int i = 0; i < N / 4; i++) {
+            const uint4 x = __ldg((const uint4 *)p + i);
+            t[4 * i] = x.x; t[4 * i + 1] = x.y; t[4 * i + 2] = x.z; t[4 * i + 3] = x.w;
+        }
+    }
+}
+__device__ __forceinline__ uint4 load4(const uint32_t *p, bool al) {
+    if (al) return *(const uint4 *)p;
+    return make_uint4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ void store4(uint32_t *p, uint4 v, bool al) {
+    if (al) { *(uint4 *)p = v; return; }
+    p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+}
+
+template <bool FWD>
+__device__ __forceinline__ void butterfly(uint32_t &a, uint32_t &b, uint32_t t2) {
+    if (FWD) {
+        const uint32_t x = mmul_t2(b, t2);
+        b = msub(a, x);
+        a = madd(a, x);
+    } else {
+        const uint32_t d = msub(a, b);
+        a = madd(a, b);
+        b = mmul_t2(d, t2);
+    }
+}
+
+// What a thread knows of its pass: column, tile and table addresses.
+struct VecCtx {
+    uint32_t hb;        // upper pass: index bits above the pass; bottom pass: the block's first element
+    uint32_t *col;      // this column + the tile's first element
+    const uint32_t *in;
+    uint32_t tid;
+    bool al, tal;       // 16-byte aligned data, tables
+    uint32_t emask;     // bottom pass: a source shorter than the block repeats
+    uint32_t n_in_tile; // bottom pass: elements of this block that exist (4096 unless the transform is shorter)
+};
+
+// Layer of index bit B on the thread's 8 groups.
+template <bool FWD, int R, int WL, int A, int B>
+__device__ __forceinline__ void vec_layer(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    constexpr int rb = B - A, RL = 4 >> rb, J = B - WL;
+    const uint32_t h = WL ? (c.hb << (R - 1 - J)) + (base >> (B + 1)) : (c.hb + base) >> (B + 1);
+    uint32_t t[RL];
+    load_run<RL>(t, p.line + p.off.v[p.s + J - 1] + h, c.tal);
+#pragma unroll
+    for (int i = 0; i < RL; i++) t[i] *= 2u;
+#pragma unroll
+    for (int i0 = 0; i0 < 8; i0++) {
+        if (i0 & (1 << rb)) continue;
+#pragma unroll
+        for (int w = 0; w < 4; w++) butterfly<FWD>(v[i0][w], v[i0 | (1 << rb)][w], t[i0 >> (rb + 1)]);
+    }
+}
+// Layers 1 and 0, within the groups of 4 words (bits [2, 5) = the 8 groups).
+template <bool FWD>
+__device__ __forceinline__ void vec_layer1(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    uint32_t t[8];
+    load_run<8>(t, p.line + p.off.v[0] + ((c.hb + base) >> 2), c.tal);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        butterfly<FWD>(v[i][0], v[i][2], 2u * t[i]);
+        butterfly<FWD>(v[i][1], v[i][3], 2u * t[i]);
+    }
+}
+template <bool FWD>
+__device__ __forceinline__ void vec_layer0(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    const uint32_t h = (c.hb + base) >> 1;  // a multiple of 16
+    if (p.cmode == 0u) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            uint32_t t[8];
+            load_run<8>(t, p.circle + h + 8 * q, c.tal);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                butterfly<FWD>(v[4 * q + i][0], v[4 * q + i][1], 2u * t[2 * i]);
+                butterfly<FWD>(v[4 * q + i][2], v[4 * q + i][3], 2u * t[2 * i + 1]);
+            }
+        }
+    } else {  // [y, -y, -x, x] of the pair (x, y) for each four twiddles (circle_tw)
+        uint32_t t[8];
+        load_run<8>(t, p.circle + (h >> 1), c.tal);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t x = t[2 * i], y = t[2 * i + 1];
+            butterfly<FWD>(v[2 * i][0], v[2 * i][1], 2u * y);
+            butterfly<FWD>(v[2 * i][2], v[2 * i][3], 2u * msub(0u, y));
+            butterfly<FWD>(v[2 * i + 1][0], v[2 * i + 1][1], 2u * msub(0u, x));
+            butterfly<FWD>(v[2 * i + 1][2], v[2 * i + 1][3], 2u * x);
+        }
+    }
+}
+
+template <bool FWD, int R, int WL, int K, int JJ>
+__device__ __forceinline__ void vec_layers(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    using St = VecStage<FWD, R, WL, K>;
+    if constexpr (JJ < St::HI - St::LO) {
+        vec_layer<FWD, R, WL, St::A, FWD ? St::HI - 1 - JJ : St::LO + JJ>(v, p, c, base);
+        vec_layers<FWD, R, WL, K, JJ + 1>(v, p, c, base);
+    }
+}
+
+// Stage K and the ones after it.
+template <bool FWD, int R, int WL, int K>
+__device__ __forceinline__ void vec_stages(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t *sm) {
+    using St = VecStage<FWD, R, WL, K>;
+    constexpr int A = St::A;
+    constexpr bool FIRST = K == 0, LAST = K + 1 == St::NST;
+    // the thread's index bits around [A, A+3) and the two low ones
+    const uint32_t base = ((c.tid & ((1u << (A - 2)) - 1u)) << 2) | ((c.tid >> (A - 2)) << (A + 3));
+    const uint32_t pb = vpad(base);
+    const bool act = WL || base < c.n_in_tile;
+    // tile index of group i -> element: rows of 2^WL words are 2^s apart
+    auto elem = [&](uint32_t e) { return WL ? ((uint64_t)(e >> WL) << p.s) | (e & ((1u << WL) - 1u)) : (uint64_t)e; };
+    const uint32_t turn = (c.tid & ~31u) * 32u + (c.tid & 31u) * 4u;  // coalesced order within a warp's 1024 words
+    if constexpr (FIRST) {
+        if constexpr (St::TURN) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t e = turn + 128u * i;
+                if (e < c.n_in_tile) *(uint4 *)(sm + vpad(e)) = load4(c.in + (e & c.emask), c.al);
+            }
+            __syncwarp();
+        } else if (act) {
+            const uint32_t *q = c.in + elem(WL ? base : base & c.emask);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint4 x = load4(q + elem((uint32_t)i << A), c.al);
+                v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+            }
+        }
+    }
+    if constexpr (!FIRST || St::TURN) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint4 x = *(const uint4 *)(sm + pb + vpad((uint32_t)i << A));
+            v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+        }
+    }
+    if (act) {
+        if constexpr (St::TURN && !FWD) {
+            vec_layer0<FWD>(v, p, c, base);
+            vec_layer1<FWD>(v, p, c, base);
+        }
+        vec_layers<FWD, R, WL, K, 0>(v, p, c, base);
+        if constexpr (St::TURN && FWD) {
+            vec_layer1<FWD>(v, p, c, base);
+            vec_layer0<FWD>(v, p, c, base);
+        }
+        if (LAST && p.scale != 1u) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int w = 0; w < 4; w++) v[i][w] = mmul_t2(v[i][w], 2u * p.scale);
+        }
+    }
+    if constexpr (LAST && !St::TURN) {
+        if (act) {
+            uint32_t *q = c.col + elem(base);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                store4(q + elem((uint32_t)i << A), make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]), c.al);
+        }
+    } else {
+        // a thread writes the words it read, so one barrier per exchange is enough
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            *(uint4 *)(sm + pb + vpad((uint32_t)i << A)) = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
+        if constexpr (LAST) {
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t e = turn + 128u * i;
+                if (e < c.n_in_tile) store4(c.col + e, *(const uint4 *)(sm + vpad(e)), c.al);
+            }
+        } else {
+            // blocks of index bits below bit 10 stay within a warp's 1024 elements
+            if constexpr (A <= 7 && VecStage<FWD, R, WL, K + 1>::A <= 7) __syncwarp();
+            else __syncthreads();
+            vec_stages<FWD, R, WL, K + 1>(v, p, c, sm);
+        }
+    }
+}
+
+// Block `tile` of 4096 elements of column `ci`.
+template <bool FWD, int R, int WL>
+__device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint32_t ci, uint32_t *sm) {
+    static_assert(WL == 0 ? (R >= 5 && R <= 12) : (R >= 3 && R + WL == 12 && WL >= 3), "vector pass shapes");
+    VecCtx c;
+    c.tid = threadIdx.x;
+    uint64_t gbase;
+    if constexpr (WL == 0) {
+        gbase = tile * kVecTile;
+        c.hb = (uint32_t)gbase;
+        c.emask = p.src && p.src_mask < kVecTile ? (uint32_t)p.src_mask : kVecTile - 1u;
+        c.n_in_tile = p.n_elems - gbase < kVecTile ? (uint32_t)(p.n_elems - gbase) : kVecTile;
+    } else {
+        // column blocks consecutive, or the replicas of an LDE's source tile (see tile_pass)
+        const uint32_t cshift = p.s - WL;
+        const uint64_t cb = p.hb_log ? tile >> p.hb_log : tile & ((1ull << cshift) - 1ull);
+        const uint64_t hb = p.hb_log ? tile & ((1ull << p.hb_log) - 1ull) : tile >> cshift;
+        gbase = (hb << (p.s + R)) | (cb << WL);
+        c.hb = (uint32_t)hb;
+        c.emask = kVecTile - 1u;
+        c.n_in_tile = kVecTile;
+    }
+    uint32_t *col = p.dev_cols ? p.dev_cols[ci] : p.data + (uint64_t)ci * p.col_stride;
+    const uint32_t *in = p.src ? p.src + (uint64_t)ci * p.src_stride : col;
+    c.al = (((uintptr_t)col | (uintptr_t)in) & 15u) == 0;
+    c.tal = (((uintptr_t)p.line | (uintptr_t)p.circle) & 15u) == 0;
+    c.col = col + gbase;
+    c.in = in + (p.src ? (gbase & p.src_mask) : gbase);
+    uint32_t v[8][4];
+    vec_stages<FWD, R, WL, 0>(v, p, c, sm);
+}
+
+template <bool FWD, int R, int WL>
+__global__ void __launch_bounds__(kVecThreads, VX_NTT_VEC_BLOCKS) ntt_vec_kernel(const __grid_constant__ Pass2Args p) {
+    __shared__ __align__(16) uint32_t sm[kVecSmemWords];
+    pdl_wait();
+    vec_pass<FWD, R, WL>(p, blockIdx.x, blockIdx.y, sm);
+}
+
 // Several transforms of different lengths in one launch: group g's columns
 // and tiles are blocks [first[g], first[g+1]) of a 1-D grid, each group with
-// its own pass shape, all on 4096-element tiles of 256 threads (bottom
-// passes of 12 layers, upper passes of 3..9).  Used for columns of uneven
-// sizes, so a small size group does not run as a launch of its own that
-// leaves most SMs idle.
+// its own pass shape (bottom passes of 11 or 12 layers, upper passes of
+// 3..9).  Used for columns of uneven sizes, so a small size group does not
+// run as a launch of its own that leaves most SMs idle.
 constexpr uint32_t kMaxNttGroups = 4;
 struct MultiPassArgs {
     Pass2Args g[kMaxNttGroups];
@@ -383,8 +667,8 @@ struct MultiPassArgs {
 };
 
 template <bool FWD>
-__global__ void __launch_bounds__(256, 4) ntt_multi_kernel(MultiPassArgs a) {
-    extern __shared__ uint32_t dsm[];
+__global__ void __launch_bounds__(kVecThreads, VX_NTT_VEC_BLOCKS) ntt_multi_kernel(const __grid_constant__ MultiPassArgs a) {
+    __shared__ __align__(16) uint32_t sm[kVecSmemWords];
     pdl_wait();
     const uint32_t b = blockIdx.x;
     uint32_t gi = 0;
@@ -394,14 +678,15 @@ __global__ void __launch_bounds__(256, 4) ntt_multi_kernel(MultiPassArgs a) {
     const uint64_t tile = local - ci * a.tiles[gi];
     const Pass2Args &p = a.g[gi];
     switch (a.R[gi]) {
-    case 12: tile_pass<FWD, 12, 0, 256>(p, tile, ci, dsm); break;
-    case 9: tile_pass<FWD, 9, 3, 256>(p, tile, ci, dsm); break;
-    case 8: tile_pass<FWD, 8, 4, 256>(p, tile, ci, dsm); break;
-    case 7: tile_pass<FWD, 7, 5, 256>(p, tile, ci, dsm); break;
-    case 6: tile_pass<FWD, 6, 6, 256>(p, tile, ci, dsm); break;
-    case 5: tile_pass<FWD, 5, 7, 256>(p, tile, ci, dsm); break;
-    case 4: tile_pass<FWD, 4, 8, 256>(p, tile, ci, dsm); break;
-    case 3: tile_pass<FWD, 3, 9, 256>(p, tile, ci, dsm); break;
+    case 12: vec_pass<FWD, 12, 0>(p, tile, ci, sm); break;
+    case 11: vec_pass<FWD, 11, 0>(p, tile, ci, sm); break;
+    case 9: vec_pass<FWD, 9, 3>(p, tile, ci, sm); break;
+    case 8: vec_pass<FWD, 8, 4>(p, tile, ci, sm); break;
+    case 7: vec_pass<FWD, 7, 5>(p, tile, ci, sm); break;
+    case 6: vec_pass<FWD, 6, 6>(p, tile, ci, sm); break;
+    case 5: vec_pass<FWD, 5, 7>(p, tile, ci, sm); break;
+    case 4: vec_pass<FWD, 4, 8>(p, tile, ci, sm); break;
+    case 3: vec_pass<FWD, 3, 9>(p, tile, ci, sm); break;
     default: break;
     }
 }
@@ -429,37 +714,44 @@ cudaError_t launch_pass2(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cu
     return launch_pdl(ntt_tile_kernel<FWD, R, WL, NT>, dim3((unsigned)tiles, n_cols), dim3(NT), smem, st, a);
 }
 
-// Pass shapes the kernels are built for (ntt_plan only emits these):
-// bottom passes (WL = 0) of 4..14 layers; upper passes of 3..9 layers on
+template <bool FWD, int R, int WL>
+cudaError_t launch_vec(const Pass2Args &a, uint32_t n_cols, cudaStream_t st) {
+    const uint64_t blocks = (a.n_elems + kVecTile - 1) / kVecTile;
+    return launch_pdl(ntt_vec_kernel<FWD, R, WL>, dim3((unsigned)blocks, n_cols), dim3(kVecThreads), 0, st, a);
+}
+
+// Pass shapes the kernels are built for (ntt_plan only emits these): bottom
+// passes (WL = 0) of 4..14 layers; upper passes of 3..9 layers on
 // 2^12-element tiles (WL = 12 - R), of 10 and 11 layers on 2^13-element
 // tiles (WL = 13 - R) and of 12 layers on 2^14-element tiles (WL = 2): rows
-// of at least 16 bytes.
+// of at least 16 bytes.  The vector pass takes bottoms of 5..12 layers and
+// uppers of 3..9; the others hold 16 elements per thread (tile_pass).
 template <bool FWD>
 cudaError_t dispatch_pass2(uint32_t r, uint32_t wl, const Pass2Args &a, uint64_t tiles, uint32_t n_cols,
                            cudaStream_t st) {
     if (wl == 0) {
         switch (r) {
         case 4: return launch_pass2<FWD, 4, 0>(a, tiles, n_cols, st);
-        case 5: return launch_pass2<FWD, 5, 0>(a, tiles, n_cols, st);
-        case 6: return launch_pass2<FWD, 6, 0>(a, tiles, n_cols, st);
-        case 7: return launch_pass2<FWD, 7, 0>(a, tiles, n_cols, st);
-        case 8: return launch_pass2<FWD, 8, 0>(a, tiles, n_cols, st);
-        case 9: return launch_pass2<FWD, 9, 0>(a, tiles, n_cols, st);
-        case 10: return launch_pass2<FWD, 10, 0>(a, tiles, n_cols, st);
-        case 11: return launch_pass2<FWD, 11, 0>(a, tiles, n_cols, st);
-        case 12: return launch_pass2<FWD, 12, 0>(a, tiles, n_cols, st);
+        case 5: return launch_vec<FWD, 5, 0>(a, n_cols, st);
+        case 6: return launch_vec<FWD, 6, 0>(a, n_cols, st);
+        case 7: return launch_vec<FWD, 7, 0>(a, n_cols, st);
+        case 8: return launch_vec<FWD, 8, 0>(a, n_cols, st);
+        case 9: return launch_vec<FWD, 9, 0>(a, n_cols, st);
+        case 10: return launch_vec<FWD, 10, 0>(a, n_cols, st);
+        case 11: return launch_vec<FWD, 11, 0>(a, n_cols, st);
+        case 12: return launch_vec<FWD, 12, 0>(a, n_cols, st);
         case 13: return launch_pass2<FWD, 13, 0>(a, tiles, n_cols, st);
         case 14: return launch_pass2<FWD, 14, 0>(a, tiles, n_cols, st);
         }
     } else if (wl + r == 12) {
         switch (r) {
-        case 3: return launch_pass2<FWD, 3, 9>(a, tiles, n_cols, st);
-        case 4: return launch_pass2<FWD, 4, 8>(a, tiles, n_cols, st);
-        case 5: return launch_pass2<FWD, 5, 7>(a, tiles, n_cols, st);
-        case 6: return launch_pass2<FWD, 6, 6>(a, tiles, n_cols, st);
-        case 7: return launch_pass2<FWD, 7, 5>(a, tiles, n_cols, st);
-        case 8: return launch_pass2<FWD, 8, 4>(a, tiles, n_cols, st);
-        case 9: return launch_pass2<FWD, 9, 3>(a, tiles, n_cols, st);
+        case 3: return launch_vec<FWD, 3, 9>(a, n_cols, st);
+        case 4: return launch_vec<FWD, 4, 8>(a, n_cols, st);
+        case 5: return launch_vec<FWD, 5, 7>(a, n_cols, st);
+        case 6: return launch_vec<FWD, 6, 6>(a, n_cols, st);
+        case 7: return launch_vec<FWD, 7, 5>(a, n_cols, st);
+        case 8: return launch_vec<FWD, 8, 4>(a, n_cols, st);
+        case 9: return launch_vec<FWD, 9, 3>(a, n_cols, st);
         }
     } else if (wl + r == 13) {
         switch (r) {
@@ -647,6 +939,7 @@ cudaError_t ntt_transform_planned(uint32_t *data, uint32_t *const *dev_cols, uin
         a.vec = (vec && (pw[i] >= 2u || ps[i] == 0u)) ? 1u : 0u;
         // the first forward pass of an LDE reads each source tile for 2^(log_n - src_log) replicas
         a.hb_log = (q == 0 && src && forward && log_n > src_log && ps[i] + pr[i] == src_log) ? log_n - src_log : 0u;
+        a.n_elems = 1ull << log_n;
         uint64_t tiles = (1ull << log_n) >> (pr[i] + pw[i]);
         e = forward ? dispatch_pass2<true>(pr[i], pw[i], a, tiles, n_cols, stream)
                     : dispatch_pass2<false>(pr[i], pw[i], a, tiles, n_cols, stream);
@@ -657,15 +950,15 @@ cudaError_t ntt_transform_planned(uint32_t *data, uint32_t *const *dev_cols, uin
 
 cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool forward, cudaStream_t stream,
                                  uint32_t *launches) {
-    // groups whose transform is exactly a 12-layer bottom pass plus one upper
-    // pass of 3..9 layers (15..21 layers) share the launches; the others run
-    // as transforms of their own
+    // groups whose transform is an 11-layer bottom pass plus one upper pass of
+    // 3..9 layers (14..20 layers), or 12 + 9 layers, share the launches; the
+    // others run as transforms of their own
     if (n_groups > 64) return cudaErrorInvalidValue;
     bool merge[64] = {false};
     uint32_t n_merge = 0;
     for (uint32_t g = 0; g < n_groups; g++) {
         const uint32_t total = (grp[g].src && forward) ? grp[g].src_log : grp[g].log_n;
-        merge[g] = n_merge < kMaxNttGroups && grp[g].n_cols > 0 && total >= 15 && total <= 21 &&
+        merge[g] = n_merge < kMaxNttGroups && grp[g].n_cols > 0 && total >= 14 && total <= 21 &&
                    !(grp[g].src && !forward && grp[g].src_log != grp[g].log_n);
         n_merge += merge[g];
     }
@@ -678,20 +971,6 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
         if (launches) *launches += ntt_pass_count((G.src && forward) ? G.src_log : G.log_n, G.log_n);
     }
     if (n_merge < 2) return cudaSuccess;
-    static bool attr_done[64] = {false};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const size_t smem = (tw_base(4096) + 4096) * 4;
-    if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-        e = cudaFuncSetAttribute(forward ? ntt_multi_kernel<true> : ntt_multi_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(forward ? ntt_multi_kernel<false> : ntt_multi_kernel<true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr_done[dev] = true;
-    }
     for (uint32_t q = 0; q < 2; q++) {
         const uint32_t pi = forward ? 1u - q : q;  // forward: the upper pass first
         MultiPassArgs a;
@@ -701,7 +980,7 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
             if (!merge[g]) continue;
             const NttGroup &G = grp[g];
             const uint32_t total = (G.src && forward) ? G.src_log : G.log_n;
-            const uint32_t r = pi == 0 ? 12u : total - 12u, wl = pi == 0 ? 0u : 12u - r;
+            const uint32_t bottom = total <= 20u ? 11u : 12u, r = pi == 0 ? bottom : total - bottom;
             const uint32_t e2 = (30u * G.log_n) % 31u;
             Pass2Args &p = a.g[a.n_groups];
             p.data = G.data; p.dev_cols = nullptr; p.col_stride = G.col_stride;
@@ -710,10 +989,9 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
             p.src_stride = G.src ? (1ull << G.src_log) : 0ull;
             p.line = G.tw.line; p.circle = G.tw.circle; p.cmode = G.tw.circle_mode;
             for (int i = 0; i < 32; i++) p.off.v[i] = G.tw.off[i];
-            p.s = pi == 0 ? 0u : 12u;
+            p.s = pi == 0 ? 0u : bottom;
+            p.n_elems = 1ull << G.log_n;
             p.scale = (!forward && q == 1u) ? (e2 == 0 ? 1u : (1u << e2)) : 1u;
-            p.vec = ((((uintptr_t)G.data & 15u) == 0) && (G.n_cols == 1 || G.col_stride % 4u == 0) &&
-                     (!G.src || ((((uintptr_t)G.src & 15u) == 0) && G.src_log >= 2))) ? 1u : 0u;
             p.hb_log = (q == 0 && G.src && forward && G.log_n > G.src_log && p.s + r == G.src_log)
                            ? G.log_n - G.src_log : 0u;
             a.R[a.n_groups] = r;
@@ -721,11 +999,10 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
             a.first[a.n_groups] = blocks;
             blocks += a.tiles[a.n_groups] * G.n_cols;
             a.n_groups++;
-            (void)wl;
         }
         a.first[a.n_groups] = blocks;
-        e = launch_pdl(forward ? ntt_multi_kernel<true> : ntt_multi_kernel<false>, dim3(blocks), dim3(256), smem,
-                       stream, a);
+        cudaError_t e = launch_pdl(forward ? ntt_multi_kernel<true> : ntt_multi_kernel<false>, dim3(blocks),
+                                   dim3(kVecThreads), 0, stream, a);
         if (e != cudaSuccess) return e;
         if (launches) *launches += 1;
     }

@@ -46,8 +46,9 @@ cudaError_t ntt_transform_planned(uint32_t *data, uint32_t *const *dev_cols, uin
 // Transforms of several column groups of different lengths, for the same
 // direction: group g is n_cols columns of 2^log_n words at data + c *
 // col_stride, with its own tables and optional source (as ntt_transform).
-// Groups of 15..21 applied layers share one launch per pass (a 12-layer
-// bottom pass and one upper pass); the others run as their own transforms.
+// Groups of 14..21 applied layers share one launch per pass (a bottom pass of
+// 11 layers, 12 for 21, and one upper pass); the others run as their own
+// transforms.
 // `launches` (if non-null) is increased by the kernels enqueued.
 struct NttGroup {
     uint32_t *data;
