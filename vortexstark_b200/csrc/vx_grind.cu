@@ -51,9 +51,64 @@ __device__ __forceinline__ uint32_t mod_p(uint32_t h) {
 // value, or from device memory when dptr is not null.
 constexpr uint32_t kPerLane = 4, kWarpChunk = 32 * kPerLane;
 
+// The nonce is message words 8 and 9 and words 10..15 are zero, so round 0's
+// column step and three of its diagonal G's are the same for every nonce:
+// they are computed once per thread.  At the other end the first digest word
+// decides almost every candidate; of the last diagonal step it needs one G
+// and three quarters of another.  70.5 of the 80 G's remain; the few
+// candidates that pass are hashed in full.
+struct GrindState { uint32_t v[16]; };
+__device__ __forceinline__ void grind_prefix(const Digest8 &d, GrindState &s) {
+    const uint32_t one = 1u;
+    uint32_t v0 = VX_IV0 ^ 0x01010020u, v1 = VX_IV1, v2 = VX_IV2, v3 = VX_IV3, v4 = VX_IV4, v5 = VX_IV5, v6 = VX_IV6,
+             v7 = VX_IV7, v8 = VX_IV0, v9 = VX_IV1, v10 = VX_IV2, v11 = VX_IV3, v12 = VX_IV4 ^ 40u, v13 = VX_IV5,
+             v14 = ~VX_IV6, v15 = VX_IV7;
+    VX_G(v0, v4, v8, v12, d.w[0], d.w[1]);
+    VX_G(v1, v5, v9, v13, d.w[2], d.w[3]);
+    VX_G(v2, v6, v10, v14, d.w[4], d.w[5]);
+    VX_G(v3, v7, v11, v15, d.w[6], d.w[7]);
+    VX_GD(v1, v6, v11, v12, 0u, 0u);
+    VX_GD(v2, v7, v8, v13, 0u, 0u);
+    VX_GD(v3, v4, v9, v14, 0u, 0u);
+    s = GrindState{{v0, v1, v2, v3, v4, v5, v6, v7, v8, v9, v10, v11, v12, v13, v14, v15}};
+}
+
+// First digest word of one nonce, from the prefix state.
+__device__ __forceinline__ uint32_t grind_word0(const Digest8 &d, const GrindState &s, uint64_t nonce, uint32_t one) {
+    uint32_t m[16];
+#pragma unroll
+    for (int i = 0; i < 8; i++) m[i] = d.w[i];
+    m[8] = (uint32_t)nonce;
+    m[9] = (uint32_t)(nonce >> 32);
+#pragma unroll
+    for (int i = 10; i < 16; i++) m[i] = 0u;
+    uint32_t v0 = s.v[0], v1 = s.v[1], v2 = s.v[2], v3 = s.v[3], v4 = s.v[4], v5 = s.v[5], v6 = s.v[6], v7 = s.v[7],
+             v8 = s.v[8], v9 = s.v[9], v10 = s.v[10], v11 = s.v[11], v12 = s.v[12], v13 = s.v[13], v14 = s.v[14],
+             v15 = s.v[15];
+    VX_GD(v0, v5, v10, v15, m[8], m[9]);
+    VX_ROUND(14, 10, 4, 8, 9, 15, 13, 6, 1, 12, 0, 2, 11, 7, 5, 3);
+    VX_ROUND(11, 8, 12, 0, 5, 2, 15, 13, 10, 14, 3, 6, 7, 1, 9, 4);
+    VX_ROUND(7, 9, 3, 1, 13, 12, 11, 14, 2, 6, 5, 10, 4, 0, 15, 8);
+    VX_ROUND(9, 0, 5, 7, 2, 4, 10, 15, 14, 1, 11, 12, 6, 8, 3, 13);
+    VX_ROUND(2, 12, 6, 10, 0, 11, 8, 3, 4, 13, 7, 5, 15, 14, 1, 9);
+    VX_ROUND(12, 5, 1, 15, 14, 13, 4, 10, 0, 7, 6, 3, 9, 2, 8, 11);
+    VX_ROUND(13, 11, 7, 14, 12, 1, 3, 9, 5, 0, 15, 4, 8, 6, 2, 10);
+    VX_ROUND(6, 15, 14, 9, 11, 3, 0, 8, 12, 2, 13, 7, 1, 4, 10, 5);
+    VX_G(v0, v4, v8, v12, m[10], m[2]);
+    VX_G(v1, v5, v9, v13, m[8], m[4]);
+    VX_G(v2, v6, v10, v14, m[7], m[6]);
+    VX_G(v3, v7, v11, v15, m[1], m[5]);
+    VX_GD(v0, v5, v10, v15, m[15], m[11]);
+    VX_GD(v2, v7, v8, v13, m[3], m[12]);
+    return (VX_IV0 ^ 0x01010020u) ^ v0 ^ v8;
+}
+
 template <bool M31OUT>
-__device__ __forceinline__ void grind_one(const Digest8 &d, unsigned long long *result, uint32_t pow_bits,
-                                          uint64_t nonce, uint32_t one) {
+__device__ __forceinline__ void grind_one(const Digest8 &d, const GrindState &s, unsigned long long *result,
+                                          uint32_t pow_bits, uint64_t nonce, uint32_t one) {
+    uint32_t w = grind_word0(d, s, nonce, one);  // one == 1: Blake2s pipe balance
+    if (M31OUT) w = mod_p(w);
+    if (w & (pow_bits >= 32u ? ~0u : (1u << pow_bits) - 1u)) return;
     uint32_t m[16];
 #pragma unroll
     for (int i = 0; i < 8; i++) m[i] = d.w[i];
@@ -62,7 +117,7 @@ __device__ __forceinline__ void grind_one(const Digest8 &d, unsigned long long *
 #pragma unroll
     for (int i = 10; i < 16; i++) m[i] = 0u;
     uint32_t h[8];
-    blake2s_block(h, m, 40u, one);  // one == 1: Blake2s pipe balance
+    blake2s_block(h, m, 40u);
     uint32_t h0 = h[0], h1 = h[1], h2 = h[2], h3 = h[3];
     if (M31OUT) { h0 = mod_p(h0); h1 = mod_p(h1); h2 = mod_p(h2); h3 = mod_p(h3); }
     if (tz128(h0, h1, h2, h3) >= pow_bits) atomicMin(result, (unsigned long long)nonce);
@@ -76,6 +131,8 @@ __global__ void __launch_bounds__(256) grind_kernel(Digest8 d, const uint32_t *d
 #pragma unroll
         for (int i = 0; i < 8; i++) d.w[i] = __ldg(dptr + i);
     }
+    GrindState pre;
+    grind_prefix(d, pre);
     const uint64_t lowmask = lowbits >= 63 ? ~0ull : ((1ull << lowbits) - 1ull);
     auto nonce_of = [&](uint64_t w) { return lowbits >= 63 ? base + w : base + ((w >> lowbits) << 32) + (w & lowmask); };
     if (next) {
@@ -94,7 +151,7 @@ __global__ void __launch_bounds__(256) grind_kernel(Digest8 d, const uint32_t *d
 #pragma unroll 1
             for (uint32_t r = 0; r < kPerLane; r++) {
                 const uint64_t w = c0 + 32u * r + lane;
-                if (w < count) grind_one<M31OUT>(d, result, pow_bits, nonce_of(w), one);
+                if (w < count) grind_one<M31OUT>(d, pre, result, pow_bits, nonce_of(w), one);
             }
         }
     }
@@ -102,7 +159,7 @@ __global__ void __launch_bounds__(256) grind_kernel(Digest8 d, const uint32_t *d
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < count; w += stride) {
         const uint64_t nonce = nonce_of(w);
         if (nonce > __ldcv(result)) return;  // a smaller nonce is already accepted
-        grind_one<M31OUT>(d, result, pow_bits, nonce, one);
+        grind_one<M31OUT>(d, pre, result, pow_bits, nonce, one);
     }
 }
 
