@@ -115,18 +115,22 @@ class MerkleTree:
         return paths
 
     @staticmethod
+    def _tile_roots(columns, n):
+        """The 1024-leaf tile roots, on the device."""
+        ptrs = _ptrs(columns)
+        sub = _empty(n // TILE_SIZE * 8)
+        _lib.lib().cuda_merkle_tiled_generic(ptrs.data_ptr(), sub.data_ptr(), len(columns), n)
+        return sub
+
+    @staticmethod
     def commit_root_only_with_subtrees(columns, log_n_leaves: int):
         """merkle.rs:386-451 — root and the 1024-leaf tile roots."""
-        L = _lib.lib()
         n = 1 << log_n_leaves
         if n < TILE_SIZE:
             t = MerkleTree.commit(columns, log_n_leaves)
             return t.root(), []
-        ptrs = _ptrs(columns)
-        tiles = n // TILE_SIZE
-        sub = _empty(tiles * 8)
-        L.cuda_merkle_tiled_generic(ptrs.data_ptr(), sub.data_ptr(), len(columns), n)
-        return MerkleTree._reduce(sub, tiles), [tuple(int(x) for x in r) for r in _words(sub).reshape(-1, 8)]
+        sub = MerkleTree._tile_roots(columns, n)
+        return MerkleTree._reduce(sub, n // TILE_SIZE), [tuple(int(x) for x in r) for r in _words(sub).reshape(-1, 8)]
 
     @staticmethod
     def commit_root_soa4_with_subtrees(c0, c1, c2, c3, log_n_leaves: int):
@@ -143,7 +147,12 @@ class MerkleTree:
 
     @staticmethod
     def commit_root_only(columns, log_n_leaves: int) -> tuple:
-        return MerkleTree.commit_root_only_with_subtrees(columns, log_n_leaves)[0]
+        """merkle.rs:142-231 — the tile roots stay on the device (as Python
+        tuples they took 5.6 of 6.0 ms at 2^22 leaves)."""
+        n = 1 << log_n_leaves
+        if n < TILE_SIZE:
+            return MerkleTree.commit(columns, log_n_leaves).root()
+        return MerkleTree._reduce(MerkleTree._tile_roots(columns, n), n // TILE_SIZE)
 
     @staticmethod
     def _reduce(cur, size: int) -> tuple:
