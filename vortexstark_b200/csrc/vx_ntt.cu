@@ -434,13 +434,27 @@ __device__ __forceinline__ void load_run(uint32_t t[N], const uint32_t *__restri
         }
     }
 }
+// Data accesses name the global space: through a generic address the compiler
+// would have to keep them in order with the shared-memory exchanges.
 __device__ __forceinline__ uint4 load4(const uint32_t *p, bool al) {
-    if (al) return *(const uint4 *)p;
-    return make_uint4(p[0], p[1], p[2], p[3]);
+    const size_t g = __cvta_generic_to_global(p);
+    uint4 v;
+    if (al) {
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(g));
+    } else {
+        asm volatile("ld.global.u32 %0, [%4];\n\tld.global.u32 %1, [%4+4];\n\tld.global.u32 %2, [%4+8];\n\t"
+                     "ld.global.u32 %3, [%4+12];"
+                     : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(g));
+    }
+    return v;
 }
 __device__ __forceinline__ void store4(uint32_t *p, uint4 v, bool al) {
-    if (al) { *(uint4 *)p = v; return; }
-    p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+    const size_t g = __cvta_generic_to_global(p);
+    if (al)
+        asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(g), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
+    else
+        asm volatile("st.global.u32 [%0], %1;\n\tst.global.u32 [%0+4], %2;\n\tst.global.u32 [%0+8], %3;\n\t"
+                     "st.global.u32 [%0+12], %4;" ::"l"(g), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
 }
 
 template <bool FWD>
@@ -467,53 +481,62 @@ struct VecCtx {
     uint32_t n_in_tile; // bottom pass: elements of this block that exist (4096 unless the transform is shorter)
 };
 
-// Layer of index bit B on the thread's 8 groups.
-template <bool FWD, int R, int WL, int A, int B>
-__device__ __forceinline__ void vec_layer(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
-    constexpr int rb = B - A, RL = 4 >> rb, J = B - WL;
+// A stage's twiddles: the run of 4 >> rb words of row bit A + rb at
+// row[(4 >> rb) - 1], and the words of layers 1 and 0.
+struct VecTw { uint32_t row[7], l1[8], l0[16]; };
+
+template <bool FWD, int R, int WL, int K, int B>
+__device__ __forceinline__ void vec_load_row(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    constexpr int RL = 4 >> (B - VecStage<FWD, R, WL, K>::A), J = B - WL;
     const uint32_t h = WL ? (c.hb << (R - 1 - J)) + (base >> (B + 1)) : (c.hb + base) >> (B + 1);
+    load_run<RL>(t.row + RL - 1, p.line + p.off.v[p.s + J - 1] + h, c.tal);
+}
+__device__ __forceinline__ void vec_load_l1(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    load_run<8>(t.l1, p.line + p.off.v[0] + ((c.hb + base) >> 2), c.tal);
+}
+// Circle twiddles h = (hb + base) / 2, a multiple of 16: 16 words, or the 8
+// words of the stwo pairs [y, -y, -x, x] (circle_tw).
+__device__ __forceinline__ void vec_load_l0(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+    const uint32_t h = (c.hb + base) >> 1;
+    load_run<8>(t.l0, p.circle + (p.cmode ? h >> 1 : h), c.tal);
+    if (!p.cmode) load_run<8>(t.l0 + 8, p.circle + h + 8, c.tal);
+}
+
+// Layer of index bit A + rb on the thread's 8 groups.
+template <bool FWD, int RB>
+__device__ __forceinline__ void vec_layer(uint32_t v[8][4], const VecTw &tw) {
+    constexpr int RL = 4 >> RB;
     uint32_t t[RL];
-    load_run<RL>(t, p.line + p.off.v[p.s + J - 1] + h, c.tal);
 #pragma unroll
-    for (int i = 0; i < RL; i++) t[i] *= 2u;
+    for (int i = 0; i < RL; i++) t[i] = 2u * tw.row[RL - 1 + i];
 #pragma unroll
     for (int i0 = 0; i0 < 8; i0++) {
-        if (i0 & (1 << rb)) continue;
+        if (i0 & (1 << RB)) continue;
 #pragma unroll
-        for (int w = 0; w < 4; w++) butterfly<FWD>(v[i0][w], v[i0 | (1 << rb)][w], t[i0 >> (rb + 1)]);
+        for (int w = 0; w < 4; w++) butterfly<FWD>(v[i0][w], v[i0 | (1 << RB)][w], t[i0 >> (RB + 1)]);
     }
 }
 // Layers 1 and 0, within the groups of 4 words (bits [2, 5) = the 8 groups).
 template <bool FWD>
-__device__ __forceinline__ void vec_layer1(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
-    uint32_t t[8];
-    load_run<8>(t, p.line + p.off.v[0] + ((c.hb + base) >> 2), c.tal);
+__device__ __forceinline__ void vec_layer1(uint32_t v[8][4], const VecTw &tw) {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        butterfly<FWD>(v[i][0], v[i][2], 2u * t[i]);
-        butterfly<FWD>(v[i][1], v[i][3], 2u * t[i]);
+        butterfly<FWD>(v[i][0], v[i][2], 2u * tw.l1[i]);
+        butterfly<FWD>(v[i][1], v[i][3], 2u * tw.l1[i]);
     }
 }
 template <bool FWD>
-__device__ __forceinline__ void vec_layer0(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
-    const uint32_t h = (c.hb + base) >> 1;  // a multiple of 16
-    if (p.cmode == 0u) {
+__device__ __forceinline__ void vec_layer0(uint32_t v[8][4], const VecTw &tw, uint32_t cmode) {
+    if (cmode == 0u) {
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            uint32_t t[8];
-            load_run<8>(t, p.circle + h + 8 * q, c.tal);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                butterfly<FWD>(v[4 * q + i][0], v[4 * q + i][1], 2u * t[2 * i]);
-                butterfly<FWD>(v[4 * q + i][2], v[4 * q + i][3], 2u * t[2 * i + 1]);
-            }
+        for (int i = 0; i < 8; i++) {
+            butterfly<FWD>(v[i][0], v[i][1], 2u * tw.l0[2 * i]);
+            butterfly<FWD>(v[i][2], v[i][3], 2u * tw.l0[2 * i + 1]);
         }
-    } else {  // [y, -y, -x, x] of the pair (x, y) for each four twiddles (circle_tw)
-        uint32_t t[8];
-        load_run<8>(t, p.circle + (h >> 1), c.tal);
+    } else {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t x = t[2 * i], y = t[2 * i + 1];
+            const uint32_t x = tw.l0[2 * i], y = tw.l0[2 * i + 1];
             butterfly<FWD>(v[2 * i][0], v[2 * i][1], 2u * y);
             butterfly<FWD>(v[2 * i][2], v[2 * i][3], 2u * msub(0u, y));
             butterfly<FWD>(v[2 * i + 1][0], v[2 * i + 1][1], 2u * msub(0u, x));
@@ -522,44 +545,89 @@ __device__ __forceinline__ void vec_layer0(uint32_t v[8][4], const Pass2Args &p,
     }
 }
 
-template <bool FWD, int R, int WL, int K, int JJ>
-__device__ __forceinline__ void vec_layers(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t base) {
+// The row layers of stage K in order, each loading its twiddles first (LOAD)
+// or finding them in tw.
+template <bool FWD, int R, int WL, int K, int JJ, bool LOAD, bool RUN>
+__device__ __forceinline__ void vec_layers(uint32_t v[8][4], VecTw &tw, const Pass2Args &p, const VecCtx &c,
+                                           uint32_t base) {
     using St = VecStage<FWD, R, WL, K>;
     if constexpr (JJ < St::HI - St::LO) {
-        vec_layer<FWD, R, WL, St::A, FWD ? St::HI - 1 - JJ : St::LO + JJ>(v, p, c, base);
-        vec_layers<FWD, R, WL, K, JJ + 1>(v, p, c, base);
+        constexpr int B = FWD ? St::HI - 1 - JJ : St::LO + JJ;
+        if constexpr (LOAD) vec_load_row<FWD, R, WL, K, B>(tw, p, c, base);
+        if constexpr (RUN) vec_layer<FWD, B - St::A>(v, tw);
+        vec_layers<FWD, R, WL, K, JJ + 1, LOAD, RUN>(v, tw, p, c, base);
     }
 }
 
-// Stage K and the ones after it.
+// The thread's index bits around [A, A+3) and the two low ones.
+template <int A>
+__device__ __forceinline__ uint32_t vec_base(uint32_t tid) {
+    return ((tid & ((1u << (A - 2)) - 1u)) << 2) | ((tid >> (A - 2)) << (A + 3));
+}
+
+// PRE: every stage's twiddles are loaded along with the data, so their latencies
+// overlap; for launches of at most four blocks per SM, where nothing else
+// hides them and registers are free (2^10 interpolate 15.8 -> 15.0 us).
 template <bool FWD, int R, int WL, int K>
-__device__ __forceinline__ void vec_stages(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c, uint32_t *sm) {
+__device__ __forceinline__ void vec_prefetch(VecTw *tw, const Pass2Args &p, const VecCtx &c) {
+    using St = VecStage<FWD, R, WL, K>;
+    if constexpr (K < St::NST) {
+        const uint32_t base = vec_base<St::A>(c.tid);
+        if (WL || base < c.n_in_tile) {
+            vec_layers<FWD, R, WL, K, 0, true, false>(nullptr, tw[K], p, c, base);
+            if constexpr (St::TURN) {
+                vec_load_l1(tw[K], p, c, base);
+                vec_load_l0(tw[K], p, c, base);
+            }
+        }
+        vec_prefetch<FWD, R, WL, K + 1>(tw, p, c);
+    }
+}
+
+// Tile index -> element: rows of 2^WL words are 2^s apart.
+template <int WL>
+__device__ __forceinline__ uint64_t vec_elem(const Pass2Args &p, uint32_t e) {
+    return WL ? ((uint64_t)(e >> WL) << p.s) | (e & ((1u << WL) - 1u)) : (uint64_t)e;
+}
+// First of a thread's 8 groups, 128 words apart, in coalesced order within its warp's 1024 words.
+__device__ __forceinline__ uint32_t vec_turn(uint32_t tid) { return (tid & ~31u) * 32u + (tid & 31u) * 4u; }
+
+// The words of the first stage, in its order or (TURN) in coalesced order.
+template <bool FWD, int R, int WL>
+__device__ __forceinline__ void vec_first(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c) {
+    using St = VecStage<FWD, R, WL, 0>;
+    const uint32_t base = vec_base<St::A>(c.tid), turn = vec_turn(c.tid);
+    const uint32_t *q = c.in + vec_elem<WL>(p, WL ? base : base & c.emask);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (St::TURN) {
+            const uint32_t e = turn + 128u * i;
+            if (e < c.n_in_tile) x = load4(c.in + (e & c.emask), c.al);
+        } else {
+            if (WL || base < c.n_in_tile) x = load4(q + vec_elem<WL>(p, (uint32_t)i << St::A), c.al);
+        }
+        v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+    }
+}
+
+// Stage K and the ones after it (the first finds its words in v).
+template <bool FWD, int R, int WL, int K, bool PRE>
+__device__ __forceinline__ void vec_stages(uint32_t v[8][4], VecTw *tw, const Pass2Args &p, const VecCtx &c,
+                                           uint32_t *sm) {
     using St = VecStage<FWD, R, WL, K>;
     constexpr int A = St::A;
     constexpr bool FIRST = K == 0, LAST = K + 1 == St::NST;
-    // the thread's index bits around [A, A+3) and the two low ones
-    const uint32_t base = ((c.tid & ((1u << (A - 2)) - 1u)) << 2) | ((c.tid >> (A - 2)) << (A + 3));
+    const uint32_t base = vec_base<A>(c.tid);
     const uint32_t pb = vpad(base);
     const bool act = WL || base < c.n_in_tile;
-    // tile index of group i -> element: rows of 2^WL words are 2^s apart
-    auto elem = [&](uint32_t e) { return WL ? ((uint64_t)(e >> WL) << p.s) | (e & ((1u << WL) - 1u)) : (uint64_t)e; };
-    const uint32_t turn = (c.tid & ~31u) * 32u + (c.tid & 31u) * 4u;  // coalesced order within a warp's 1024 words
-    if constexpr (FIRST) {
-        if constexpr (St::TURN) {
+    auto elem = [&](uint32_t e) { return vec_elem<WL>(p, e); };
+    const uint32_t turn = vec_turn(c.tid);
+    if constexpr (FIRST && St::TURN) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t e = turn + 128u * i;
-                if (e < c.n_in_tile) *(uint4 *)(sm + vpad(e)) = load4(c.in + (e & c.emask), c.al);
-            }
-            __syncwarp();
-        } else if (act) {
-            const uint32_t *q = c.in + elem(WL ? base : base & c.emask);
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint4 x = load4(q + elem((uint32_t)i << A), c.al);
-                v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
-            }
-        }
+        for (int i = 0; i < 8; i++)
+            *(uint4 *)(sm + vpad(turn + 128u * i)) = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
+        __syncwarp();
     }
     if constexpr (!FIRST || St::TURN) {
 #pragma unroll
@@ -569,14 +637,19 @@ __device__ __forceinline__ void vec_stages(uint32_t v[8][4], const Pass2Args &p,
         }
     }
     if (act) {
+        VecTw &t = tw[PRE ? K : 0];
         if constexpr (St::TURN && !FWD) {
-            vec_layer0<FWD>(v, p, c, base);
-            vec_layer1<FWD>(v, p, c, base);
+            if constexpr (!PRE) vec_load_l0(t, p, c, base);
+            vec_layer0<FWD>(v, t, p.cmode);
+            if constexpr (!PRE) vec_load_l1(t, p, c, base);
+            vec_layer1<FWD>(v, t);
         }
-        vec_layers<FWD, R, WL, K, 0>(v, p, c, base);
+        vec_layers<FWD, R, WL, K, 0, !PRE, true>(v, t, p, c, base);
         if constexpr (St::TURN && FWD) {
-            vec_layer1<FWD>(v, p, c, base);
-            vec_layer0<FWD>(v, p, c, base);
+            if constexpr (!PRE) vec_load_l1(t, p, c, base);
+            vec_layer1<FWD>(v, t);
+            if constexpr (!PRE) vec_load_l0(t, p, c, base);
+            vec_layer0<FWD>(v, t, p.cmode);
         }
         if (LAST && p.scale != 1u) {
 #pragma unroll
@@ -599,22 +672,25 @@ __device__ __forceinline__ void vec_stages(uint32_t v[8][4], const Pass2Args &p,
             *(uint4 *)(sm + pb + vpad((uint32_t)i << A)) = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
         if constexpr (LAST) {
             __syncwarp();
+            uint4 x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = *(const uint4 *)(sm + vpad(turn + 128u * i));
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const uint32_t e = turn + 128u * i;
-                if (e < c.n_in_tile) store4(c.col + e, *(const uint4 *)(sm + vpad(e)), c.al);
+                if (e < c.n_in_tile) store4(c.col + e, x[i], c.al);
             }
         } else {
             // blocks of index bits below bit 10 stay within a warp's 1024 elements
             if constexpr (A <= 7 && VecStage<FWD, R, WL, K + 1>::A <= 7) __syncwarp();
             else __syncthreads();
-            vec_stages<FWD, R, WL, K + 1>(v, p, c, sm);
+            vec_stages<FWD, R, WL, K + 1, PRE>(v, tw, p, c, sm);
         }
     }
 }
 
 // Block `tile` of 4096 elements of column `ci`.
-template <bool FWD, int R, int WL>
+template <bool FWD, int R, int WL, bool PRE = false>
 __device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint32_t ci, uint32_t *sm) {
     static_assert(WL == 0 ? (R >= 5 && R <= 12) : (R >= 3 && R + WL == 12 && WL >= 3), "vector pass shapes");
     VecCtx c;
@@ -642,14 +718,19 @@ __device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint
     c.col = col + gbase;
     c.in = in + (p.src ? (gbase & p.src_mask) : gbase);
     uint32_t v[8][4];
-    vec_stages<FWD, R, WL, 0>(v, p, c, sm);
+    VecTw tw[PRE ? VecStage<FWD, R, WL, 0>::NST : 1];
+    vec_first<FWD, R, WL>(v, p, c);
+    if constexpr (PRE) vec_prefetch<FWD, R, WL, 0>(tw, p, c);
+    vec_stages<FWD, R, WL, 0, PRE>(v, tw, p, c, sm);
 }
 
-template <bool FWD, int R, int WL>
-__global__ void __launch_bounds__(kVecThreads, VX_NTT_VEC_BLOCKS) ntt_vec_kernel(const __grid_constant__ Pass2Args p) {
+constexpr uint32_t kVecPreBlocks = 4;
+template <bool FWD, int R, int WL, bool PRE>
+__global__ void __launch_bounds__(kVecThreads, PRE ? kVecPreBlocks : VX_NTT_VEC_BLOCKS)
+    ntt_vec_kernel(const __grid_constant__ Pass2Args p) {
     __shared__ __align__(16) uint32_t sm[kVecSmemWords];
     pdl_wait();
-    vec_pass<FWD, R, WL>(p, blockIdx.x, blockIdx.y, sm);
+    vec_pass<FWD, R, WL, PRE>(p, blockIdx.x, blockIdx.y, sm);
 }
 
 // Several transforms of different lengths in one launch: group g's columns
@@ -714,44 +795,57 @@ cudaError_t launch_pass2(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cu
     return launch_pdl(ntt_tile_kernel<FWD, R, WL, NT>, dim3((unsigned)tiles, n_cols), dim3(NT), smem, st, a);
 }
 
+// The vector pass, or the 16-element one where a launch is too short for it:
+// from 2^11 to below 2^20 elements the chip is not full either way, and twice
+// the threads with half the work each finish first (launcher times, 2^16:
+// 18.8 us against 19.0 forward and 19.4 inverse; 2^19: 20.4 against 21.0 and
+// 22.0; 2^20: 25.1 against 24.5 and 25.0; 2^22: 43.6 against 37.6).  Columns
+// behind a device pointer array stay with the vector pass, whose accesses are
+// 16 bytes wide there too (8 x 2^14: 22.0 against 21.3 us).
 template <bool FWD, int R, int WL>
-cudaError_t launch_vec(const Pass2Args &a, uint32_t n_cols, cudaStream_t st) {
+cudaError_t launch_pass(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cudaStream_t st) {
+    const uint64_t total = a.n_elems * n_cols;
+    if (!a.dev_cols && total >= (1ull << 11) && total < (1ull << 20))
+        return launch_pass2<FWD, R, WL>(a, tiles, n_cols, st);
     const uint64_t blocks = (a.n_elems + kVecTile - 1) / kVecTile;
-    return launch_pdl(ntt_vec_kernel<FWD, R, WL>, dim3((unsigned)blocks, n_cols), dim3(kVecThreads), 0, st, a);
+    const dim3 grid((unsigned)blocks, n_cols);
+    if (blocks * n_cols <= 148u * kVecPreBlocks)
+        return launch_pdl(ntt_vec_kernel<FWD, R, WL, true>, grid, dim3(kVecThreads), 0, st, a);
+    return launch_pdl(ntt_vec_kernel<FWD, R, WL, false>, grid, dim3(kVecThreads), 0, st, a);
 }
 
 // Pass shapes the kernels are built for (ntt_plan only emits these): bottom
 // passes (WL = 0) of 4..14 layers; upper passes of 3..9 layers on
 // 2^12-element tiles (WL = 12 - R), of 10 and 11 layers on 2^13-element
 // tiles (WL = 13 - R) and of 12 layers on 2^14-element tiles (WL = 2): rows
-// of at least 16 bytes.  The vector pass takes bottoms of 5..12 layers and
-// uppers of 3..9; the others hold 16 elements per thread (tile_pass).
+// of at least 16 bytes.  Bottoms of 5..12 layers and uppers of 3..9 have the
+// vector pass; the others run as tile_pass.
 template <bool FWD>
 cudaError_t dispatch_pass2(uint32_t r, uint32_t wl, const Pass2Args &a, uint64_t tiles, uint32_t n_cols,
                            cudaStream_t st) {
     if (wl == 0) {
         switch (r) {
         case 4: return launch_pass2<FWD, 4, 0>(a, tiles, n_cols, st);
-        case 5: return launch_vec<FWD, 5, 0>(a, n_cols, st);
-        case 6: return launch_vec<FWD, 6, 0>(a, n_cols, st);
-        case 7: return launch_vec<FWD, 7, 0>(a, n_cols, st);
-        case 8: return launch_vec<FWD, 8, 0>(a, n_cols, st);
-        case 9: return launch_vec<FWD, 9, 0>(a, n_cols, st);
-        case 10: return launch_vec<FWD, 10, 0>(a, n_cols, st);
-        case 11: return launch_vec<FWD, 11, 0>(a, n_cols, st);
-        case 12: return launch_vec<FWD, 12, 0>(a, n_cols, st);
+        case 5: return launch_pass<FWD, 5, 0>(a, tiles, n_cols, st);
+        case 6: return launch_pass<FWD, 6, 0>(a, tiles, n_cols, st);
+        case 7: return launch_pass<FWD, 7, 0>(a, tiles, n_cols, st);
+        case 8: return launch_pass<FWD, 8, 0>(a, tiles, n_cols, st);
+        case 9: return launch_pass<FWD, 9, 0>(a, tiles, n_cols, st);
+        case 10: return launch_pass<FWD, 10, 0>(a, tiles, n_cols, st);
+        case 11: return launch_pass<FWD, 11, 0>(a, tiles, n_cols, st);
+        case 12: return launch_pass<FWD, 12, 0>(a, tiles, n_cols, st);
         case 13: return launch_pass2<FWD, 13, 0>(a, tiles, n_cols, st);
         case 14: return launch_pass2<FWD, 14, 0>(a, tiles, n_cols, st);
         }
     } else if (wl + r == 12) {
         switch (r) {
-        case 3: return launch_vec<FWD, 3, 9>(a, n_cols, st);
-        case 4: return launch_vec<FWD, 4, 8>(a, n_cols, st);
-        case 5: return launch_vec<FWD, 5, 7>(a, n_cols, st);
-        case 6: return launch_vec<FWD, 6, 6>(a, n_cols, st);
-        case 7: return launch_vec<FWD, 7, 5>(a, n_cols, st);
-        case 8: return launch_vec<FWD, 8, 4>(a, n_cols, st);
-        case 9: return launch_vec<FWD, 9, 3>(a, n_cols, st);
+        case 3: return launch_pass<FWD, 3, 9>(a, tiles, n_cols, st);
+        case 4: return launch_pass<FWD, 4, 8>(a, tiles, n_cols, st);
+        case 5: return launch_pass<FWD, 5, 7>(a, tiles, n_cols, st);
+        case 6: return launch_pass<FWD, 6, 6>(a, tiles, n_cols, st);
+        case 7: return launch_pass<FWD, 7, 5>(a, tiles, n_cols, st);
+        case 8: return launch_pass<FWD, 8, 4>(a, tiles, n_cols, st);
+        case 9: return launch_pass<FWD, 9, 3>(a, tiles, n_cols, st);
         }
     } else if (wl + r == 13) {
         switch (r) {
