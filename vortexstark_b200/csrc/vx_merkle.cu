@@ -65,7 +65,9 @@ uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf
     uint32_t h = 0;
     lv->top = 0;
     if (depth > 16) {
-        h = (leaf_k >= 1 && leaf_k <= 4) ? leaf_k : tree_leaf_k(depth);  // leaf kernel: 2^h leaves per thread
+        // leaf kernel: 2^h leaves per thread; without a device's choice, at
+        // least 2^16 threads
+        h = (leaf_k >= 1 && leaf_k <= 4) ? leaf_k : (depth < 21 ? (depth > 18 ? depth - 17 : 1u) : 4u);
         add(h);
         // node kernels, at most 16 -> 1, down to 2^16 hashes.  A thread of a
         // node kernel keeps every lane busy; the reduce launch, with a block
