@@ -31,10 +31,11 @@ struct LeafFold {
     }
 };
 
-// The last FRI layers, of at most 2^kTailLog values each, in one single-block
-// launch: fold, tree and transcript step of every layer, with the folded
-// values, messages and transcript state in shared memory.
-constexpr uint32_t kTailLog = 8;
+// The last FRI layers, of at most 2^kTailLog values each, in one launch: fold,
+// tree and transcript step of every layer, with the folded values, messages
+// and transcript state in shared memory.  Layers of up to 2^kTailBlockLog
+// values run in one block, larger ones in a cluster of kTailCluster.
+constexpr uint32_t kTailLog = 11, kTailBlockLog = 8, kTailCluster = 8;
 struct FriTailLayer {
     const uint32_t *tw;
     uint32_t *out[4];
