@@ -167,13 +167,27 @@ __global__ void __launch_bounds__(256) combine_groups_kernel(const __grid_consta
 #pragma unroll
             for (int c = 0; c < 4; c++) s[k][c] = fold64(s[k][c]);
     };
+    // the next three columns are on their way while three are accumulated
     uint32_t j = 0;
+    uint4 v[3];
+    if (cnt >= 3u) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i] = __ldg(cp + i * cs4);
+    }
     for (; j + 3u <= cnt; j += 3u) {
-        const uint4 v0 = __ldg(cp + j * cs4), v1 = __ldg(cp + (j + 1u) * cs4), v2 = __ldg(cp + (j + 2u) * cs4);
-        mac(v0, spw[first + j]);
-        mac(v1, spw[first + j + 1u]);
-        mac(v2, spw[first + j + 2u]);
+        uint4 w[3];
+        const bool more = j + 6u <= cnt;
+        if (more) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) w[i] = __ldg(cp + (j + 3u + i) * cs4);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) mac(v[i], spw[first + j + i]);
         fold();
+        if (more) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) v[i] = w[i];
+        }
     }
     for (; j < cnt; j++) mac(__ldg(cp + j * cs4), spw[first + j]);  // at most two more
     fold();
