@@ -89,6 +89,17 @@ __device__ __forceinline__ uint32_t dot4(uint32_t m0, uint32_t z0, uint32_t m1, 
                                          uint32_t m3, uint32_t z3) {
     return reduce64((uint64_t)m0 * z0 + (uint64_t)m1 * z1 + (uint64_t)m2 * z2 + (uint64_t)m3 * z3);
 }
+// x + y + m z for canonical x, y, z, the sums in the same 64-bit accumulators:
+// 4 (P - 1)^2 + 2 (P - 1) < 2^64.
+__device__ __forceinline__ qm31 qadd2_mul_mat(qm31 x, qm31 y, const qmat &m, qm31 z) {
+    const uint32_t z0 = z.v[0], z1 = z.v[1], z2 = z.v[2], z3 = z.v[3];
+    auto dot = [&](int i, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+        return reduce64((uint64_t)(x.v[i] + y.v[i]) + (uint64_t)m0 * z0 + (uint64_t)m1 * z1 + (uint64_t)m2 * z2 +
+                        (uint64_t)m3 * z3);
+    };
+    return {{dot(0, m.a0, m.na1, m.c0, m.nc1), dot(1, m.a1, m.a0, m.c1, m.c0), dot(2, m.a2, m.na3, m.a0, m.na1),
+             dot(3, m.a3, m.a2, m.a1, m.a0)}};
+}
 __device__ __forceinline__ qm31 qmul_mat(const qmat &m, qm31 z) {
     const uint32_t z0 = z.v[0], z1 = z.v[1], z2 = z.v[2], z3 = z.v[3];
     return {{dot4(m.a0, z0, m.na1, z1, m.c0, z2, m.nc1, z3), dot4(m.a1, z0, m.a0, z1, m.c1, z2, m.c0, z3),

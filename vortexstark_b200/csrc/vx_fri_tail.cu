@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kReduceThreads) fri_tail_kernel(const __grid_c
         uint32_t *cur = buf[0], *nxt = buf[1];
         if (tid < n) {
             const qmat am = qmat_of(qm31{{al[0], al[1], al[2], al[3]}});
-            const qm31 r = qadd(qadd(f0, f1), qmul_mat(am, qmulm(qsub(f0, f1), tw)));
+            const qm31 r = qadd2_mul_mat(f0, f1, am, qmulm(qsub(f0, f1), tw));
 #pragma unroll
             for (int c = 0; c < 4; c++) L.out[c][first + tid] = r.v[c];
             vals[k & 1][tid] = make_uint4(r.v[0], r.v[1], r.v[2], r.v[3]);
