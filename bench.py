@@ -285,17 +285,17 @@ def served_benchmark(seed: int, n_requests: int = 512, policy=None):
 # DRAM bytes of one LDE (iNTT 2^24 + evaluate 2^26) at log_n = 24 from an ncu
 # capture of the current kernels (dram__bytes_read.sum + dram__bytes_write.sum
 # of the LDE's pass launches); None until measured.
-LDE_TRAFFIC_LOG24 = 1141.03e6 + 673.23e6
+LDE_TRAFFIC_LOG24 = 1141.07e6 + 671.70e6
 LDE_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the LDE's six pass launches (plans "
                       "11 + 7 + 6 each way), one proof slot at log_n = 24, one-pass metrics: "
-                      "profiles/ntt_tile_lde_log24.md. The bottom evaluate pass reads its twiddles, as large as "
+                      "profiles/ntt_vec_lde_log24.md. The bottom evaluate pass reads its twiddles, as large as "
                       "the data")
 
 # DRAM bytes of the trace commitment at log_n = 24 (2^26 leaves: leaf subtrees,
-# 16 -> 1 nodes, reduce) from an ncu capture of one proof slot.
-TRACE_COMMIT_TRAFFIC_LOG24 = (269.08e6 + 176.44e6) + (142.33e6 + 18.59e6) + (8.46e6 + 0.0)
-TRACE_COMMIT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the trace commitment's three launches "
-                               "(leaf_subtree_kernel<LeafM31>, node_subtree_kernel, tree_reduce_kernel<LeafM31>), one "
+# nodes, reduce) from an ncu capture of one proof slot.
+TRACE_COMMIT_TRAFFIC_LOG24 = (269.68e6 + 176.98e6) + (142.14e6 + 18.34e6) + (8.41e6 + 0.0) + (2.17e6 + 0.0)
+TRACE_COMMIT_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the trace commitment's four launches "
+                               "(leaf_subtree_kernel<LeafM31>, node_subtree_kernel twice, tree_reduce_kernel<LeafM31>), one "
                                "proof slot at log_n = 24, one-pass metrics: profiles/merkle_trace_commit_log24.md. "
                                "Reads: the 2^26 leaf words once, then the stored level of 2^22 hashes")
 
