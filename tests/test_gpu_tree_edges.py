@@ -30,6 +30,45 @@ def test_roots_at_every_depth(oracle, log_n, ncols):
             tune.set_leaf_k(log_n, 0)
 
 
+def _least_words(depth, k=4):
+    """Words of the plan that stores least: 2^k-leaf subtrees, 16 -> 1 node
+    levels while more than 2^20 hashes are left, every 4th height above."""
+    heights = [k]
+    while depth - heights[-1] > 20:
+        heights.append(heights[-1] + 4)
+    left = max(depth - heights[-1] - 8, 0)
+    while heights[-1] < depth:
+        heights.append(min(heights[-1] + 4, depth))
+    counters = 0
+    while left > 0:
+        step = min(left, 8)
+        counters += 1 << (left - step)
+        left -= step
+    return sum(8 << (depth - h) for h in heights) + counters
+
+
+@pytest.mark.parametrize("log_n", [17, 18, 20, 21, 22, 23, 24, 25, 26])
+def test_root_in_a_small_workspace(oracle, log_n):
+    """A workspace of the least words of that plan is enough (some depths take less)."""
+    import ctypes as C
+
+    import torch
+
+    from vortexstark_b200 import _lib
+    col = m31_array(7 + log_n, 1 << log_n)
+    want = tuple(oracle.merkle_root([col]).tolist())
+    d = to_dev(col)
+    ptrs = (C.c_void_p * 1)(d.data_ptr())
+    words = _least_words(log_n)
+    work = torch.empty(words, dtype=torch.int32, device="cuda")
+    root = torch.empty(8, dtype=torch.int32, device="cuda")
+    call = _lib.lib().vx_merkle_root_cols
+    assert call(ptrs, 1, log_n, work.data_ptr(), words, root.data_ptr(), None) == 0
+    assert tuple(int(x) for x in root.cpu().numpy().view(np.uint32)) == want
+    assert call(ptrs, 1, log_n, work.data_ptr(), words // 2, root.data_ptr(), None) == 1
+    _lib.clear_error()
+
+
 @pytest.mark.parametrize("log_n,blowup,nq", [(4, 1, 1), (4, 1, 3), (4, 3, 17), (5, 2, 4), (6, 3, 5), (7, 2, 33),
                                              (8, 1, 2), (9, 1, 31), (10, 2, 79), (11, 3, 1), (13, 1, 7), (15, 3, 81)])
 def test_proofs_at_odd_query_counts(oracle, log_n, blowup, nq):

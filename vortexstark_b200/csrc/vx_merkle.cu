@@ -51,7 +51,7 @@ uint32_t tree_leaf_k(uint32_t depth, uint32_t kind) {
     return (uint32_t)(k < 1 ? 1 : (k > 4 ? 4 : k));
 }
 
-uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf_k) {
+uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf_k, uint32_t reduce_log) {
     lv->n = 1;
     lv->height[0] = 0;
     lv->hashes[0] = nullptr;
@@ -73,7 +73,7 @@ uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf
         // node kernel keeps every lane busy; the reduce launch, with a block
         // of 256 threads per 256 hashes and half of them idle a level later,
         // takes over where its chain of levels, not the hashing, sets the time.
-        while (depth - h > kReduceLog) { h += depth - h - kReduceLog < 4 ? depth - h - kReduceLog : 4; add(h); }
+        while (depth - h > reduce_log) { h += depth - h - reduce_log < 4 ? depth - h - reduce_log : 4; add(h); }
         lv->top = lv->n - 1;
     }
     // reduce stages of 8 levels from h: every 4th height is stored, so the
@@ -94,9 +94,9 @@ uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf
     return used;
 }
 
-uint64_t tree_pool_words(uint32_t depth, uint32_t leaf_k) {
+uint64_t tree_pool_words(uint32_t depth, uint32_t leaf_k, uint32_t reduce_log) {
     TreeLevels lv;
-    return tree_plan(depth, nullptr, &lv, leaf_k);
+    return tree_plan(depth, nullptr, &lv, leaf_k, reduce_log);
 }
 
 cudaError_t tree_reset(const TreeLevels &lv, cudaStream_t stream) {
@@ -161,16 +161,24 @@ extern "C" int vx_merkle_root_cols(const uint32_t *const *host_col_ptrs, uint32_
     VX_CHECK_ARG(workspace && root_out, "vx_merkle_root_cols: null workspace or root");
     for (uint32_t c = 0; c < n_cols; c++) VX_CHECK_ARG(host_col_ptrs[c], "vx_merkle_root_cols: column %u is null", c);
     const uint32_t d = log_n_leaves;
-    // the device's leaf-kernel shape, or a larger subtree (smaller stored
-    // level) if the workspace was sized for one
-    uint32_t k = tree_leaf_k(d);
-    while (k < 4 && tree_pool_words(d, k) > workspace_words) k++;
-    VX_CHECK_ARG(tree_pool_words(d, k) <= workspace_words,
-                 "vx_merkle_root_cols: workspace of %llu words, %llu needed", (unsigned long long)workspace_words,
-                 (unsigned long long)tree_pool_words(d, k));
+    // the device's leaf-kernel shape, or what stores less: a larger subtree
+    // (smaller first level), then a reduce launch over up to 2^20 hashes, with
+    // node kernels of 16 -> 1 only (no level between)
+    const uint32_t k0 = tree_leaf_k(d);
+    uint32_t k = k0, rl = kReduceLog;
+    auto fits = [&]() { return tree_pool_words(d, k, rl) <= workspace_words; };
+    while (k < 4 && !fits()) k++;
+    if (!fits()) {
+        rl = 0;
+        for (uint32_t t = 20; t >= 17 && !rl; t--)  // 2^t hashes left by 16 -> 1 steps from height k
+            for (k = k0; k <= 4 && !rl; k++)
+                if (d > 16 && tree_pool_words(d, k, t) <= workspace_words) { rl = t; break; }
+    }
+    VX_CHECK_ARG(rl != 0, "vx_merkle_root_cols: workspace of %llu words, %llu needed",
+                 (unsigned long long)workspace_words, (unsigned long long)tree_pool_words(d, k0));
     cudaStream_t st = (cudaStream_t)stream;
     TreeLevels lv;
-    tree_plan(d, workspace, &lv, k);
+    tree_plan(d, workspace, &lv, k, rl);
     VX_CUDA_TRY(tree_reset(lv, st));
     const ChanStep none{nullptr, nullptr, nullptr};
     cudaError_t e;

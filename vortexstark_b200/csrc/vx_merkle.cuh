@@ -389,8 +389,11 @@ constexpr uint32_t kReduceLog = 16;      // the reduce launch starts from at mos
 // with the leaf kernel hashing 2^leaf_k leaves per thread (1..4; 0 = the
 // current device's choice, tree_leaf_k).  A layout that sizes a pool and
 // carves it later passes the same leaf_k to both calls.
-uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf_k);
-uint64_t tree_pool_words(uint32_t depth, uint32_t leaf_k);
+// reduce_log: the reduce launch starts from at most 2^reduce_log hashes
+// (kReduceLog; up to 20 works and stores less).
+uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf_k,
+                   uint32_t reduce_log = kReduceLog);
+uint64_t tree_pool_words(uint32_t depth, uint32_t leaf_k, uint32_t reduce_log = kReduceLog);
 // Leaf-kernel subtree size (log2 of leaves per thread) for trees of this
 // depth on the current device, and the autotuner's override (1..4; 0 resets),
 // per leaf kind: narrow leaves (a few M31 words: trace columns, the quotient)

@@ -1108,7 +1108,7 @@ void prover_footprint(uint32_t log_n, uint32_t blowup, uint32_t nq, size_t *slot
     uint64_t n = 1ull << log_n, N = 1ull << le;
     uint64_t w = align_words(n) + align_words(N);
     for (uint32_t k = 0; k < L.nfri; k++) w += 4 * align_words(1ull << (le - 1 - k));
-    w += 2 * align_words(tree_pool_words(le, 0));
+    w += 2 * align_words(tree_pool_words(le, tree_leaf_k(le)));
     for (uint32_t k = 0; k < L.nfri; k++) w += align_words(tree_pool_words(le - 1 - k, tree_leaf_k(le - 1 - k, kLeafFold)));
     w += align_words(sizeof(DevChannel) / 4 + 1) + align_words(4) + align_words(4ull * (L.nfri + 1)) +
          align_words(nq) + align_words(L.words);
