@@ -3,8 +3,9 @@
 The reduce launch hashes a level of 128 nodes by threads and smaller ones by
 quads of lanes, in stages of 8 levels over blocks of 256; deeper trees start
 with leaf subtrees and node kernels down to 2^16 hashes.  Openings take eight
-lanes per (query, stored-level group), four pairs per warp, and the line folds
-of at most 256 values run in one block."""
+lanes per (query, stored-level group), four pairs per warp.  The line folds of
+at most 2048 values share one launch: a cluster of eight blocks down to 512
+values, one block from 256."""
 import numpy as np
 import pytest
 
@@ -74,3 +75,22 @@ def test_root_in_a_small_workspace(oracle, log_n):
 def test_proofs_at_odd_query_counts(oracle, log_n, blowup, nq):
     a, b = 1000 + log_n, 77 * nq
     assert prover.prove_bytes(a, b, log_n, blowup, nq) == oracle.prove(a, b, log_n, blowup, nq)
+
+
+@pytest.mark.parametrize("log_n,first", [(8, 8), (9, 9), (10, 10), (11, 11), (14, 11)])
+def test_fri_tails_while_the_device_is_full(oracle, log_n, first):
+    """Tails that start at 2^first values (above 2^8: on a cluster), several at
+    once beside larger proofs, so that a cluster's blocks start when others
+    leave room for them."""
+    import torch
+    assert first == min(log_n, 11)
+    jobs = [(log_n, 40 + i, 3 * i) for i in range(6)] + [(18, 7, 9), (18, 8, 10)]
+    work = [(prover.ProverCache(k), torch.cuda.Stream(), k, a, b) for k, a, b in jobs]
+    want = [oracle.prove(a, b, k) for k, a, b in jobs]
+    for _ in range(4):
+        for cache, stream, _, a, b in reversed(work):
+            cache.prove_async(a, b, stream.cuda_stream)
+        torch.cuda.synchronize()
+        assert [w[0].result_bytes() for w in work] == want
+    for w in work:
+        w[0].close()

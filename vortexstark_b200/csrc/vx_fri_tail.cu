@@ -11,7 +11,10 @@
 // eighth of a layer folds from the same eighth of the one before, so values
 // stay in their block; the eight subtree roots go to block 0's shared memory,
 // which finishes the tree and the transcript step and sends the challenge to
-// every block.
+// every block.  Shared memory of another block may be written only once that
+// block runs: every block arrives at the cluster barrier first of all and
+// waits for the others right before its first remote store, so the wait is
+// over by then and costs nothing on the chain.
 #include <cooperative_groups.h>
 
 #include "vx_common.cuh"
@@ -30,10 +33,12 @@ __global__ void __launch_bounds__(kReduceThreads) fri_tail_kernel(const __grid_c
     __shared__ __align__(16) uint32_t roots[2][8 * kMsgWords];
     __shared__ uint4 vals[2][1 << kTailBlockLog];
     __shared__ uint32_t al[4];
+    cg::cluster_group cl = cg::this_cluster();
+    bool split = a.d0 > kTailBlockLog;
+    if (split) cl.barrier_arrive();  // this block has started; the wait is before the first remote store
     Quad q;
     q.init();
     pdl_wait();
-    cg::cluster_group cl = cg::this_cluster();
     const uint32_t rank = blockIdx.x;  // one cluster per launch
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     uint32_t s0 = 0, s1 = 0;
@@ -51,7 +56,6 @@ __global__ void __launch_bounds__(kReduceThreads) fri_tail_kernel(const __grid_c
             f0.v[c] = x.x; f1.v[c] = x.y;
         }
     };
-    bool split = a.d0 > kTailBlockLog;
     uint32_t m = 1u << a.d0;                                  // values of the layer
     uint32_t n = split ? m / kTailCluster : m;                // of which this block's
     uint32_t first = split ? rank * n : 0u;
@@ -103,6 +107,7 @@ __global__ void __launch_bounds__(kReduceThreads) fri_tail_kernel(const __grid_c
             // subtree roots at height d - 3 -> block 0
             uint32_t h = 0;
             while ((n >> h) > 1u) h++;
+            if (k == 0) cl.barrier_wait();
             if (tid < 4) {
                 uint32_t *d = cl.map_shared_rank(&roots[0][0], 0) + kMsgWords * (rank >> 1) + 8u * (rank & 1u) + tid;
                 d[0] = o0; d[4] = o1;
