@@ -60,3 +60,35 @@ def test_columns_of_mixed_alignment(oracle, log_n):
     ntt.interpolate_stwo_batch(d, stw)
     for c, t in zip(cols, d):
         assert np.array_equal(to_host(t), c)
+
+
+def _repacked(cache, gap):
+    """The line tables with `gap` unused words ahead of every layer."""
+    offs = [o + (i + 1) * gap for i, o in enumerate(cache.layer_offsets)]
+    for name in ("d_twiddles", "d_itwiddles"):
+        old = to_host(getattr(cache, name))
+        new = np.full(len(old) + gap * len(offs), 0x7FFFFFFE, dtype=np.uint32)
+        for o, p, n in zip(cache.layer_offsets, offs, cache.layer_sizes):
+            new[p:p + n] = old[o:o + n]
+        setattr(cache, name, to_dev(new))
+    cache.layer_offsets = offs
+
+
+@pytest.mark.parametrize("gap", [1, 2, 3, 4])
+@pytest.mark.parametrize("log_n", [4, 5, 8, 10, 12, 14, 17, 21, 22])
+def test_layer_offsets_of_the_caller(oracle, log_n, gap):
+    """Layers at word offsets that no wide load may start at."""
+    coset = Coset.half_coset(log_n)
+    oc = oracle.coset("half_coset", log_n)
+    cache = ntt.TwiddleCache(coset)
+    _repacked(cache, gap)
+    cols = [m31_array(70 + log_n + c, 1 << log_n) for c in range(2)]
+    evs = [oracle.ntt_evaluate(c, oc) for c in cols]
+    d = [to_dev(c) for c in cols]
+    ntt.evaluate(d[0], cache)
+    assert np.array_equal(to_host(d[0]), evs[0])
+    ntt.interpolate(d[0], cache)
+    ntt.evaluate_batch(d, cache)
+    assert all(np.array_equal(to_host(x), e) for x, e in zip(d, evs))
+    ntt.interpolate_batch(d, cache)
+    assert all(np.array_equal(to_host(x), c) for x, c in zip(d, cols))

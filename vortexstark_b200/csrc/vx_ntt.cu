@@ -123,6 +123,7 @@ struct Pass2Args {
     uint32_t vec;     // 1: columns and source 16-byte aligned, 4 consecutive elements per access
     uint32_t hb_log;  // > 0: the 2^hb_log tiles that read the same source tile are consecutive blocks
     uint64_t n_elems; // words per column
+    uint32_t tal;     // 1: the pass's twiddle runs allow load_run's wide loads (tables_aligned)
 };
 
 // Butterfly products: with a doubled twiddle (mmul_t2: one multiply, one
@@ -417,7 +418,7 @@ struct VecStage {
     static constexpr bool TURN = WL == 0 && A == 2;  // 32 consecutive words per thread
 };
 
-// N consecutive words from p (N-aligned index), as wide as `al` allows.
+// N consecutive words from p; `al`: p lies a multiple of min(4, N) words from a 16-byte boundary.
 template <int N>
 __device__ __forceinline__ void load_run(uint32_t t[N], const uint32_t *__restrict__ p, bool al) {
     if (N == 1 || !al) {
@@ -714,7 +715,7 @@ __device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint
     uint32_t *col = p.dev_cols ? p.dev_cols[ci] : p.data + (uint64_t)ci * p.col_stride;
     const uint32_t *in = p.src ? p.src + (uint64_t)ci * p.src_stride : col;
     c.al = (((uintptr_t)col | (uintptr_t)in) & 15u) == 0;
-    c.tal = (((uintptr_t)p.line | (uintptr_t)p.circle) & 15u) == 0;
+    c.tal = p.tal != 0u;
     c.col = col + gbase;
     c.in = in + (p.src ? (gbase & p.src_mask) : gbase);
     uint32_t v[8][4];
@@ -962,6 +963,22 @@ void ntt_knobs_get(uint32_t total, uint32_t *bottom, uint32_t *upper) {
 }
 
 namespace {
+// Whether every twiddle run of the layers [s, s + r) may be read with
+// load_run's wide loads.  A run of a layer of m twiddles is min(4, m) of its
+// words at a multiple of that, so beside the table's base the layer's own
+// offset has to be such a multiple: it is in the tables built here, but a
+// caller of the reference's launchers passes its own.
+uint32_t tables_aligned(const NttTables &tw, uint32_t log_n, uint32_t s, uint32_t r) {
+    uintptr_t base = (uintptr_t)tw.line;
+    if (s == 0) base |= (uintptr_t)tw.circle;
+    if (base & 15u) return 0;
+    for (uint32_t j = s ? s : 1u; j < s + r; j++) {
+        const uint64_t m = 1ull << (log_n - 1 - j);
+        if (tw.off[j - 1] & (uint32_t)((m < 4 ? m : 4) - 1)) return 0;
+    }
+    return 1;
+}
+
 // The knobs are looked up by the transform's length in elements (2^log_n),
 // which sets its memory regime (an LDE applies 24 layers to 2^26 elements
 // in HBM, an interpolation of 2^24 elements stays in L2), and applied to
@@ -1034,6 +1051,7 @@ cudaError_t ntt_transform_planned(uint32_t *data, uint32_t *const *dev_cols, uin
         // the first forward pass of an LDE reads each source tile for 2^(log_n - src_log) replicas
         a.hb_log = (q == 0 && src && forward && log_n > src_log && ps[i] + pr[i] == src_log) ? log_n - src_log : 0u;
         a.n_elems = 1ull << log_n;
+        a.tal = tables_aligned(tw, log_n, ps[i], pr[i]);
         uint64_t tiles = (1ull << log_n) >> (pr[i] + pw[i]);
         e = forward ? dispatch_pass2<true>(pr[i], pw[i], a, tiles, n_cols, stream)
                     : dispatch_pass2<false>(pr[i], pw[i], a, tiles, n_cols, stream);
@@ -1085,6 +1103,7 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
             for (int i = 0; i < 32; i++) p.off.v[i] = G.tw.off[i];
             p.s = pi == 0 ? 0u : bottom;
             p.n_elems = 1ull << G.log_n;
+            p.tal = tables_aligned(G.tw, G.log_n, p.s, r);
             p.scale = (!forward && q == 1u) ? (e2 == 0 ? 1u : (1u << e2)) : 1u;
             p.hb_log = (q == 0 && G.src && forward && G.log_n > G.src_log && p.s + r == G.src_log)
                            ? G.log_n - G.src_log : 0u;
