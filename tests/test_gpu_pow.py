@@ -74,3 +74,30 @@ def test_reference_launchers_match_oracle_and_reference_kernels(oracle, m31):
         if R is not None:
             rfn = R.cuda_grind_pow_m31_output if m31 else R.cuda_grind_pow
             assert _batch(rfn, pre_dev, bits, 0, 1 << 20) == want
+
+
+@pytest.mark.parametrize("m31", [False, True])
+@pytest.mark.parametrize("bits", [2, 3, 4, 6, 7, 8])
+def test_few_bits(oracle, bits, m31):
+    """Searches where most warps hold an accepted candidate at once."""
+    for seed in range(8):
+        pre = _channel(40 + seed).pow_prefix(bits)
+        assert grind_prefixed(pre, bits, m31) == oracle.grind_pow(pre, bits, m31), seed
+
+
+@pytest.mark.parametrize("m31", [False, True])
+def test_bits_around_the_first_word(oracle, m31):
+    """The first digest word decides up to 32 bits, the whole digest above.  At
+    2^31 candidates and more the answer is checked as accepted and by windows
+    around it; with a word of 31 bits (m31) 31 zeros mean a zero word."""
+    L = _lib.lib()
+    fn = L.cuda_grind_pow_m31_output if m31 else L.cuda_grind_pow
+    pre = _channel(60).pow_prefix(31)
+    n = grind_prefixed(pre, 31, m31)
+    assert oracle.verify_pow_nonce(pre, 31, n, m31)
+    pre_dev = to_dev(np.array(pre, np.uint32))
+    for bits in (29, 30, 31, 32, 33, 34):
+        want = n if oracle.verify_pow_nonce(pre, bits, n, m31) else (1 << 64) - 1
+        assert _batch(fn, pre_dev, bits, n, 1) == want, bits
+    assert _batch(fn, pre_dev, 31, n + 1, 1) == (1 << 64) - 1
+    assert _batch(fn, pre_dev, 31, max(n - 100, 0), 200) == n

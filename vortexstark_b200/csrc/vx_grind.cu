@@ -54,9 +54,11 @@ constexpr uint32_t kPerLane = 4, kWarpChunk = 32 * kPerLane;
 // The nonce is message words 8 and 9 and words 10..15 are zero, so round 0's
 // column step and three of its diagonal G's are the same for every nonce:
 // they are computed once per thread.  At the other end the first digest word
-// decides almost every candidate; of the last diagonal step it needs one G
-// and three quarters of another.  70.5 of the 80 G's remain; the few
-// candidates that pass are hashed in full.
+// decides a candidate of up to 32 bits; of the last diagonal step it needs one
+// G and three quarters of another.  70.5 of the 80 G's remain.  Above 32 bits
+// the few candidates that pass are hashed in full.  (Hashing them at every
+// number of bits costs a second compression in most warps of a search for few
+// bits: 5 bits, 70 us a search against 57.)
 struct GrindState { uint32_t v[16]; };
 __device__ __forceinline__ void grind_prefix(const Digest8 &d, GrindState &s) {
     const uint32_t one = 1u;
@@ -109,18 +111,21 @@ __device__ __forceinline__ void grind_one(const Digest8 &d, const GrindState &s,
     uint32_t w = grind_word0(d, s, nonce, one);  // one == 1: Blake2s pipe balance
     if (M31OUT) w = mod_p(w);
     if (w & (pow_bits >= 32u ? ~0u : (1u << pow_bits) - 1u)) return;
-    uint32_t m[16];
+    if (pow_bits > 32u) {
+        uint32_t m[16];
 #pragma unroll
-    for (int i = 0; i < 8; i++) m[i] = d.w[i];
-    m[8] = (uint32_t)nonce;
-    m[9] = (uint32_t)(nonce >> 32);
+        for (int i = 0; i < 8; i++) m[i] = d.w[i];
+        m[8] = (uint32_t)nonce;
+        m[9] = (uint32_t)(nonce >> 32);
 #pragma unroll
-    for (int i = 10; i < 16; i++) m[i] = 0u;
-    uint32_t h[8];
-    blake2s_block(h, m, 40u);
-    uint32_t h0 = h[0], h1 = h[1], h2 = h[2], h3 = h[3];
-    if (M31OUT) { h0 = mod_p(h0); h1 = mod_p(h1); h2 = mod_p(h2); h3 = mod_p(h3); }
-    if (tz128(h0, h1, h2, h3) >= pow_bits) atomicMin(result, (unsigned long long)nonce);
+        for (int i = 10; i < 16; i++) m[i] = 0u;
+        uint32_t h[8];
+        blake2s_block(h, m, 40u);
+        uint32_t h0 = h[0], h1 = h[1], h2 = h[2], h3 = h[3];
+        if (M31OUT) { h0 = mod_p(h0); h1 = mod_p(h1); h2 = mod_p(h2); h3 = mod_p(h3); }
+        if (tz128(h0, h1, h2, h3) < pow_bits) return;
+    }
+    atomicMin(result, (unsigned long long)nonce);
 }
 
 template <bool M31OUT>
