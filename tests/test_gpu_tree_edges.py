@@ -11,7 +11,7 @@ import pytest
 
 from gpu_util import to_dev
 from vortexstark_b200 import prover, tune
-from vortexstark_b200.merkle import FusedRoot
+from vortexstark_b200.merkle import FusedRoot, MerkleTree
 from vortexstark_b200.workload import m31_array
 
 pytestmark = pytest.mark.gpu
@@ -29,6 +29,13 @@ def test_roots_at_every_depth(oracle, log_n, ncols):
             assert FusedRoot(log_n).commit(d) == want, k
         finally:
             tune.set_leaf_k(log_n, 0)
+
+
+@pytest.mark.parametrize("ncols", [1, 4, 7])
+@pytest.mark.parametrize("log_n", [1, 5, 9, 10, 11, 14, 20, 21])
+def test_root_only_through_the_launchers(oracle, log_n, ncols):
+    cols = [m31_array(17 * log_n + i, 1 << log_n) for i in range(ncols)]
+    assert MerkleTree.commit_root_only([to_dev(c) for c in cols], log_n) == tuple(oracle.merkle_root(cols).tolist())
 
 
 def _least_words(depth, k=4):

@@ -112,3 +112,45 @@ def test_package_imports_no_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h")):
                 txt = open(os.path.join(dirpath, f)).read()
                 assert "from oracle" not in txt and "import oracle" not in txt and "vx_oracle" not in txt, f
+
+
+@pytest.mark.parametrize("call", ["commit_root_only", "commit_root_only_with_subtrees"])
+def test_column_pointers_outlive_the_launch(monkeypatch, call):
+    """The tile kernel reads the pointer array after its launch returned: the
+    array is not given back before the root has been read."""
+    import weakref
+
+    from vortexstark_b200 import merkle
+
+    class Buf:
+        def __init__(self, n=1):
+            self.n = n
+
+        def data_ptr(self):
+            return 16
+
+        def __getitem__(self, sl):
+            return self
+
+    made, alive = [], []
+
+    def ptrs(cols):
+        b = Buf()
+        made.append(weakref.ref(b))
+        return b
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: alive.append((name, made[0]() is not None))
+
+    def words(t):
+        alive.append(("read", made[0]() is not None))
+        return np.zeros(8, np.uint32)
+
+    monkeypatch.setattr(merkle, "_ptrs", ptrs)
+    monkeypatch.setattr(merkle, "_empty", Buf)
+    monkeypatch.setattr(merkle, "_words", words)
+    monkeypatch.setattr(merkle._lib, "lib", Lib)
+    getattr(merkle.MerkleTree, call)([Buf()], 22)
+    assert [n for n, _ in alive][:2] == ["cuda_merkle_tiled_generic", "cuda_merkle_hash_nodes"]
+    assert ("read", True) in alive and all(a for _, a in alive)

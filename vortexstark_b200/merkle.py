@@ -116,11 +116,12 @@ class MerkleTree:
 
     @staticmethod
     def _tile_roots(columns, n):
-        """The 1024-leaf tile roots, on the device."""
+        """The 1024-leaf tile roots, on the device, and the column pointers,
+        which the launched kernel reads: keep them until a result is back."""
         ptrs = _ptrs(columns)
         sub = _empty(n // TILE_SIZE * 8)
         _lib.lib().cuda_merkle_tiled_generic(ptrs.data_ptr(), sub.data_ptr(), len(columns), n)
-        return sub
+        return sub, ptrs
 
     @staticmethod
     def commit_root_only_with_subtrees(columns, log_n_leaves: int):
@@ -129,7 +130,7 @@ class MerkleTree:
         if n < TILE_SIZE:
             t = MerkleTree.commit(columns, log_n_leaves)
             return t.root(), []
-        sub = MerkleTree._tile_roots(columns, n)
+        sub, _keep = MerkleTree._tile_roots(columns, n)
         return MerkleTree._reduce(sub, n // TILE_SIZE), [tuple(int(x) for x in r) for r in _words(sub).reshape(-1, 8)]
 
     @staticmethod
@@ -152,7 +153,8 @@ class MerkleTree:
         n = 1 << log_n_leaves
         if n < TILE_SIZE:
             return MerkleTree.commit(columns, log_n_leaves).root()
-        return MerkleTree._reduce(MerkleTree._tile_roots(columns, n), n // TILE_SIZE)
+        sub, _keep = MerkleTree._tile_roots(columns, n)
+        return MerkleTree._reduce(sub, n // TILE_SIZE)
 
     @staticmethod
     def _reduce(cur, size: int) -> tuple:
