@@ -448,8 +448,9 @@ int vx_probe_blake2s(uint32_t blocks, uint32_t threads, uint32_t iters, uint32_t
  * stored levels' heights (heights[0] = 0 is the leaf level, the last is
  * depth); the reduce kernel starts from stored level *top (0: the leaves);
  * *n_counters group counters, *pool_words device words for the stored levels
- * and counters.  The leaf kernel's subtree size is the device-independent one;
- * vx_tune_get gives a device's. */
+ * and counters.  The leaf kernel's subtree size is the current device's for
+ * narrow leaves (vx_tune_get kind 1), so this is the plan that is built there;
+ * without a device it is a default of the host. */
 int vx_tree_plan(uint32_t depth, uint32_t heights[12], uint32_t *n_levels, uint32_t *top, uint32_t *n_counters,
                  uint64_t *pool_words);
 

@@ -9,6 +9,7 @@ values, one block from 256."""
 import numpy as np
 import pytest
 
+import test_tree_plan as tree_plan
 from gpu_util import to_dev
 from vortexstark_b200 import prover, tune
 from vortexstark_b200.merkle import FusedRoot, MerkleTree
@@ -36,6 +37,27 @@ def test_roots_at_every_depth(oracle, log_n, ncols):
 def test_root_only_through_the_launchers(oracle, log_n, ncols):
     cols = [m31_array(17 * log_n + i, 1 << log_n) for i in range(ncols)]
     assert MerkleTree.commit_root_only([to_dev(c) for c in cols], log_n) == tuple(oracle.merkle_root(cols).tolist())
+
+
+def test_the_plan_is_the_one_that_is_built():
+    """vx_tree_plan describes this device's trees, with its own rule and with a
+    subtree size that was set, and every such plan holds."""
+    from vortexstark_b200 import _lib
+    for depth in range(1, 32):
+        for k in (0, 1, 2, 3, 4):
+            tune.set_leaf_k(depth, k)
+            try:
+                heights, top, n_cnt, words = tree_plan.plan(depth)
+                assert words == _lib.lib().vx_merkle_workspace_words(depth)
+                if depth > 16:
+                    assert heights[1] == tune.get(tune.LEAF_K, depth)[0] == (k or min(max(depth - 18, 1), 4))
+                if k == 0:
+                    tree_plan.test_tree_plan_shape(depth)
+                tree_plan.check_levels(depth)
+                if 16 <= depth <= 22:
+                    tree_plan.simulate_reduce(depth, heights, top, n_cnt, k)
+            finally:
+                tune.set_leaf_k(depth, 0)
 
 
 def _least_words(depth, k=4):

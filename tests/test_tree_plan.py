@@ -98,3 +98,21 @@ def test_tree_plan_rejects_bad_depth():
     for d in (0, 32):
         with pytest.raises(_lib.VortexError):
             plan(d)
+
+
+def check_levels(depth):
+    """The reduce launch starts from at most 2^16 hashes, and the index by which
+    it finds a stored level (stored_node) is that level's."""
+    heights, top, _, _ = plan(depth)
+    assert depth - heights[top] <= 16
+    for h in range(heights[top] + 1, depth + 1):
+        u = h - heights[top]
+        if u % 4 == 0 or h == depth:
+            assert heights[top + (u + 3) // 4] == h
+        else:
+            assert h not in heights
+
+
+@pytest.mark.parametrize("depth", list(range(1, 32)))
+def test_reduce_levels(depth):
+    check_levels(depth)

@@ -34,7 +34,7 @@ void tree_knob_set(int dev, uint32_t depth, uint32_t k, uint32_t kind) {
 
 uint32_t tree_leaf_k(uint32_t depth, uint32_t kind) {
     int dev = 0;
-    cudaGetDevice(&dev);
+    const bool device = cudaGetDevice(&dev) == cudaSuccess;
     if (kind >= kLeafKinds) kind = kLeafNarrow;
     if (dev >= 0 && dev < 64 && g_leaf_k_init[dev] && depth < 32 && g_leaf_k[dev][kind][depth])
         return g_leaf_k[dev][kind][depth];
@@ -42,12 +42,14 @@ uint32_t tree_leaf_k(uint32_t depth, uint32_t kind) {
     // thread, so more threads keep their loads in flight (measured on a
     // 2^26-point FRI chain: 6.08 ms against 6.82 ms with 16 per thread).
     if (kind == kLeafFold) return 2u;
-    // narrow leaves: 2^k leaves per thread, k = 1..4, at least 2^18 threads
-    // (7 warps per SM sub-partition) before a thread takes more: the last
-    // wave of few long-running blocks costs more than the larger stored level
-    // (2^20 leaves: 108 us with 4 per thread, 118 us with 8; 2^21: 185 us
-    // with 8, 205 us with 16; 2^22 and deeper: 16 is as good or better)
-    int k = (int)depth - 18;
+    // Narrow leaves: 2^k leaves per thread, k = 1..4.  A device keeps at least
+    // 2^18 threads (14 warps per SM sub-partition of 148 SMs) before a thread
+    // takes more than two leaves: the last wave of few long-running blocks
+    // costs more than the larger stored level (2^20 leaves: 108 us with 4 per
+    // thread, 118 us with 8; 2^21: 185 us with 8, 205 us with 16; 2^22 and
+    // deeper: 16 is as good or better).  Without a device (a plan asked for on
+    // the host alone) the floor is 2^17 threads.
+    const int k = (int)depth - (device ? 18 : 17);
     return (uint32_t)(k < 1 ? 1 : (k > 4 ? 4 : k));
 }
 
@@ -65,9 +67,7 @@ uint64_t tree_plan(uint32_t depth, uint32_t *pool, TreeLevels *lv, uint32_t leaf
     uint32_t h = 0;
     lv->top = 0;
     if (depth > 16) {
-        // leaf kernel: 2^h leaves per thread; without a device's choice, at
-        // least 2^16 threads
-        h = (leaf_k >= 1 && leaf_k <= 4) ? leaf_k : (depth < 21 ? (depth > 18 ? depth - 17 : 1u) : 4u);
+        h = (leaf_k >= 1 && leaf_k <= 4) ? leaf_k : tree_leaf_k(depth);  // leaf kernel: 2^h leaves per thread
         add(h);
         // node kernels, at most 16 -> 1, down to 2^16 hashes.  A thread of a
         // node kernel keeps every lane busy; the reduce launch, with a block

@@ -364,7 +364,7 @@ __device__ __forceinline__ uint32_t chan_commit_quad(const Quad &q, const ChanSt
 //
 // Build: trees of depth <= 16 go to one multi-block reduce launch straight
 // from the leaves.  Deeper trees: one thread per 2^k-leaf subtree (k = 1..4,
-// chosen so that at least 2^16 threads run), then node kernels of at most
+// tree_leaf_k), then node kernels of at most
 // 16 -> 1 down to 2^16 hashes, then the reduce launch for the rest.
 // The reduce kernel works in stages of up to 8 levels: each block reduces 256
 // hashes in shared memory, one compression per thread per level; the last
