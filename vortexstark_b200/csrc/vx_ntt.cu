@@ -122,6 +122,11 @@ struct Pass2Args {
     uint32_t scale;   // output scale (1 = none)
     uint32_t vec;     // 1: columns and source 16-byte aligned, 4 consecutive elements per access
     uint32_t hb_log;  // > 0: the 2^hb_log tiles that read the same source tile are consecutive blocks
+};
+// What the vector pass needs beside it.  The 16-element pass is launched with
+// the above alone: 216 bytes of parameters; with these 232 a transform of
+// 2^11 to 2^19 elements took 0.3-0.5 us longer (2^14: 17.1 against 17.6 us).
+struct VecArgs : Pass2Args {
     uint64_t n_elems; // words per column
     uint32_t tal;     // 1: the pass's twiddle runs allow load_run's wide loads (tables_aligned)
 };
@@ -487,17 +492,17 @@ struct VecCtx {
 struct VecTw { uint32_t row[7], l1[8], l0[16]; };
 
 template <bool FWD, int R, int WL, int K, int B>
-__device__ __forceinline__ void vec_load_row(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+__device__ __forceinline__ void vec_load_row(VecTw &t, const VecArgs &p, const VecCtx &c, uint32_t base) {
     constexpr int RL = 4 >> (B - VecStage<FWD, R, WL, K>::A), J = B - WL;
     const uint32_t h = WL ? (c.hb << (R - 1 - J)) + (base >> (B + 1)) : (c.hb + base) >> (B + 1);
     load_run<RL>(t.row + RL - 1, p.line + p.off.v[p.s + J - 1] + h, c.tal);
 }
-__device__ __forceinline__ void vec_load_l1(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+__device__ __forceinline__ void vec_load_l1(VecTw &t, const VecArgs &p, const VecCtx &c, uint32_t base) {
     load_run<8>(t.l1, p.line + p.off.v[0] + ((c.hb + base) >> 2), c.tal);
 }
 // Circle twiddles h = (hb + base) / 2, a multiple of 16: 16 words, or the 8
 // words of the stwo pairs [y, -y, -x, x] (circle_tw).
-__device__ __forceinline__ void vec_load_l0(VecTw &t, const Pass2Args &p, const VecCtx &c, uint32_t base) {
+__device__ __forceinline__ void vec_load_l0(VecTw &t, const VecArgs &p, const VecCtx &c, uint32_t base) {
     const uint32_t h = (c.hb + base) >> 1;
     load_run<8>(t.l0, p.circle + (p.cmode ? h >> 1 : h), c.tal);
     if (!p.cmode) load_run<8>(t.l0 + 8, p.circle + h + 8, c.tal);
@@ -549,7 +554,7 @@ __device__ __forceinline__ void vec_layer0(uint32_t v[8][4], const VecTw &tw, ui
 // The row layers of stage K in order, each loading its twiddles first (LOAD)
 // or finding them in tw.
 template <bool FWD, int R, int WL, int K, int JJ, bool LOAD, bool RUN>
-__device__ __forceinline__ void vec_layers(uint32_t v[8][4], VecTw &tw, const Pass2Args &p, const VecCtx &c,
+__device__ __forceinline__ void vec_layers(uint32_t v[8][4], VecTw &tw, const VecArgs &p, const VecCtx &c,
                                            uint32_t base) {
     using St = VecStage<FWD, R, WL, K>;
     if constexpr (JJ < St::HI - St::LO) {
@@ -570,7 +575,7 @@ __device__ __forceinline__ uint32_t vec_base(uint32_t tid) {
 // overlap; for launches of at most four blocks per SM, where nothing else
 // hides them and registers are free (2^10 interpolate 15.8 -> 15.0 us).
 template <bool FWD, int R, int WL, int K>
-__device__ __forceinline__ void vec_prefetch(VecTw *tw, const Pass2Args &p, const VecCtx &c) {
+__device__ __forceinline__ void vec_prefetch(VecTw *tw, const VecArgs &p, const VecCtx &c) {
     using St = VecStage<FWD, R, WL, K>;
     if constexpr (K < St::NST) {
         const uint32_t base = vec_base<St::A>(c.tid);
@@ -587,7 +592,7 @@ __device__ __forceinline__ void vec_prefetch(VecTw *tw, const Pass2Args &p, cons
 
 // Tile index -> element: rows of 2^WL words are 2^s apart.
 template <int WL>
-__device__ __forceinline__ uint64_t vec_elem(const Pass2Args &p, uint32_t e) {
+__device__ __forceinline__ uint64_t vec_elem(const VecArgs &p, uint32_t e) {
     return WL ? ((uint64_t)(e >> WL) << p.s) | (e & ((1u << WL) - 1u)) : (uint64_t)e;
 }
 // First of a thread's 8 groups, 128 words apart, in coalesced order within its warp's 1024 words.
@@ -595,7 +600,7 @@ __device__ __forceinline__ uint32_t vec_turn(uint32_t tid) { return (tid & ~31u)
 
 // The words of the first stage, in its order or (TURN) in coalesced order.
 template <bool FWD, int R, int WL>
-__device__ __forceinline__ void vec_first(uint32_t v[8][4], const Pass2Args &p, const VecCtx &c) {
+__device__ __forceinline__ void vec_first(uint32_t v[8][4], const VecArgs &p, const VecCtx &c) {
     using St = VecStage<FWD, R, WL, 0>;
     const uint32_t base = vec_base<St::A>(c.tid), turn = vec_turn(c.tid);
     const uint32_t *q = c.in + vec_elem<WL>(p, WL ? base : base & c.emask);
@@ -614,7 +619,7 @@ __device__ __forceinline__ void vec_first(uint32_t v[8][4], const Pass2Args &p, 
 
 // Stage K and the ones after it (the first finds its words in v).
 template <bool FWD, int R, int WL, int K, bool PRE>
-__device__ __forceinline__ void vec_stages(uint32_t v[8][4], VecTw *tw, const Pass2Args &p, const VecCtx &c,
+__device__ __forceinline__ void vec_stages(uint32_t v[8][4], VecTw *tw, const VecArgs &p, const VecCtx &c,
                                            uint32_t *sm) {
     using St = VecStage<FWD, R, WL, K>;
     constexpr int A = St::A;
@@ -692,7 +697,7 @@ __device__ __forceinline__ void vec_stages(uint32_t v[8][4], VecTw *tw, const Pa
 
 // Block `tile` of 4096 elements of column `ci`.
 template <bool FWD, int R, int WL, bool PRE = false>
-__device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint32_t ci, uint32_t *sm) {
+__device__ __forceinline__ void vec_pass(const VecArgs &p, uint64_t tile, uint32_t ci, uint32_t *sm) {
     static_assert(WL == 0 ? (R >= 5 && R <= 12) : (R >= 3 && R + WL == 12 && WL >= 3), "vector pass shapes");
     VecCtx c;
     c.tid = threadIdx.x;
@@ -728,7 +733,7 @@ __device__ __forceinline__ void vec_pass(const Pass2Args &p, uint64_t tile, uint
 constexpr uint32_t kVecPreBlocks = 4;
 template <bool FWD, int R, int WL, bool PRE>
 __global__ void __launch_bounds__(kVecThreads, PRE ? kVecPreBlocks : VX_NTT_VEC_BLOCKS)
-    ntt_vec_kernel(const __grid_constant__ Pass2Args p) {
+    ntt_vec_kernel(const __grid_constant__ VecArgs p) {
     __shared__ __align__(16) uint32_t sm[kVecSmemWords];
     pdl_wait();
     vec_pass<FWD, R, WL, PRE>(p, blockIdx.x, blockIdx.y, sm);
@@ -741,7 +746,7 @@ __global__ void __launch_bounds__(kVecThreads, PRE ? kVecPreBlocks : VX_NTT_VEC_
 // run as a launch of its own that leaves most SMs idle.
 constexpr uint32_t kMaxNttGroups = 4;
 struct MultiPassArgs {
-    Pass2Args g[kMaxNttGroups];
+    VecArgs g[kMaxNttGroups];
     uint32_t R[kMaxNttGroups];
     uint32_t first[kMaxNttGroups + 1];
     uint32_t tiles[kMaxNttGroups];  // tiles per column
@@ -758,7 +763,7 @@ __global__ void __launch_bounds__(kVecThreads, VX_NTT_VEC_BLOCKS) ntt_multi_kern
     const uint32_t local = b - a.first[gi];
     const uint32_t ci = local / a.tiles[gi];
     const uint64_t tile = local - ci * a.tiles[gi];
-    const Pass2Args &p = a.g[gi];
+    const VecArgs &p = a.g[gi];
     switch (a.R[gi]) {
     case 12: vec_pass<FWD, 12, 0>(p, tile, ci, sm); break;
     case 11: vec_pass<FWD, 11, 0>(p, tile, ci, sm); break;
@@ -804,7 +809,7 @@ cudaError_t launch_pass2(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cu
 // behind a device pointer array stay with the vector pass, whose accesses are
 // 16 bytes wide there too (8 x 2^14: 22.0 against 21.3 us).
 template <bool FWD, int R, int WL>
-cudaError_t launch_pass(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cudaStream_t st) {
+cudaError_t launch_pass(const VecArgs &a, uint64_t tiles, uint32_t n_cols, cudaStream_t st) {
     const uint64_t total = a.n_elems * n_cols;
     if (!a.dev_cols && total >= (1ull << 11) && total < (1ull << 20))
         return launch_pass2<FWD, R, WL>(a, tiles, n_cols, st);
@@ -822,7 +827,7 @@ cudaError_t launch_pass(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cud
 // of at least 16 bytes.  Bottoms of 5..12 layers and uppers of 3..9 have the
 // vector pass; the others run as tile_pass.
 template <bool FWD>
-cudaError_t dispatch_pass2(uint32_t r, uint32_t wl, const Pass2Args &a, uint64_t tiles, uint32_t n_cols,
+cudaError_t dispatch_pass2(uint32_t r, uint32_t wl, const VecArgs &a, uint64_t tiles, uint32_t n_cols,
                            cudaStream_t st) {
     if (wl == 0) {
         switch (r) {
@@ -1040,7 +1045,7 @@ cudaError_t ntt_transform_planned(uint32_t *data, uint32_t *const *dev_cols, uin
                      (!src || ((((uintptr_t)src & 15u) == 0) && src_log >= 2 && (n_cols == 1 || src_stride % 4u == 0)));
     for (uint32_t q = 0; q < np; q++) {
         uint32_t i = forward ? np - 1u - q : q;   // forward: top pass first
-        Pass2Args a;
+        VecArgs a;
         a.data = data; a.dev_cols = dev_cols; a.col_stride = col_stride;
         a.src = (q == 0 && src) ? src : nullptr;
         a.src_mask = mask; a.src_stride = src_stride;
@@ -1094,7 +1099,7 @@ cudaError_t ntt_transform_groups(const NttGroup *grp, uint32_t n_groups, bool fo
             const uint32_t total = (G.src && forward) ? G.src_log : G.log_n;
             const uint32_t bottom = total <= 20u ? 11u : 12u, r = pi == 0 ? bottom : total - bottom;
             const uint32_t e2 = (30u * G.log_n) % 31u;
-            Pass2Args &p = a.g[a.n_groups];
+            VecArgs &p = a.g[a.n_groups];
             p.data = G.data; p.dev_cols = nullptr; p.col_stride = G.col_stride;
             p.src = (q == 0 && G.src) ? G.src : nullptr;
             p.src_mask = G.src ? ((1ull << G.src_log) - 1ull) : ~0ull;
