@@ -801,6 +801,21 @@ cudaError_t launch_pass2(const Pass2Args &a, uint64_t tiles, uint32_t n_cols, cu
     return launch_pdl(ntt_tile_kernel<FWD, R, WL, NT>, dim3((unsigned)tiles, n_cols), dim3(NT), smem, st, a);
 }
 
+// SMs of the current device (148 if it cannot be asked).
+uint32_t sm_count() {
+    static uint32_t cached[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148u;
+    if (!cached[dev]) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = 148;
+        }
+        cached[dev] = (uint32_t)n;
+    }
+    return cached[dev];
+}
+
 // The vector pass, or the 16-element one where a launch is too short for it:
 // from 2^11 (inverse: 2^10) to below 2^20 elements the chip is not full either
 // way, and twice the threads with half the work each finish first.  Launcher
@@ -821,7 +836,7 @@ cudaError_t launch_pass(const VecArgs &a, uint64_t tiles, uint32_t n_cols, cudaS
     const uint64_t blocks = (a.n_elems + kVecTile - 1) / kVecTile;
     const dim3 grid((unsigned)blocks, n_cols);
     if constexpr (FWD || (WL == 0 && R <= 10))
-        if ((FWD || a.n_elems <= 1024u) && blocks * n_cols <= 148u * kVecPreBlocks)
+        if ((FWD || a.n_elems <= 1024u) && blocks * n_cols <= sm_count() * kVecPreBlocks)
             return launch_pdl(ntt_vec_kernel<FWD, R, WL, true>, grid, dim3(kVecThreads), 0, st, a);
     return launch_pdl(ntt_vec_kernel<FWD, R, WL, false>, grid, dim3(kVecThreads), 0, st, a);
 }
