@@ -18,6 +18,9 @@ queries and decommitment, on the device.
            plain one-at-a-time path, swept over arrival rates, compared by
            the rate each sustains at common p99 bounds.
 
+The line holds the figures of every leg; ``--full`` prints their whole objects
+(sweeps, work, sources) in their place.
+
 N > 1 (torchrun): independent replicas, one per GPU, no collective on the
 data path ("replicas only"); barrier + max-over-ranks timing.
 ``--impl reference`` times the CPU oracle (a C restatement of the reference's
@@ -1058,6 +1061,85 @@ def blake2s_probe_rate(stream) -> float:
     return 148 * 8 * 256 * iters / (pa.elapsed_time(pb) / 1e3)
 
 
+def _rounded(x):
+    """Floats to six significant digits, in nested dicts and lists."""
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    return [_rounded(v) for v in x] if isinstance(x, list) else x
+
+
+def _timed_leaves(d, path=()):
+    """(path, dict) of every timed measurement in a microbench object."""
+    for k, v in d.items():
+        if isinstance(v, dict):
+            if "ms" in v:
+                yield path + (k,), v
+            yield from _timed_leaves(v, path + (k,))
+
+
+def _flags(d):
+    """Every equality or validity flag of a nested object."""
+    for k, v in d.items():
+        if isinstance(v, dict):
+            yield from _flags(v)
+        elif isinstance(v, bool) and ("equal" in k or k == "valid"):
+            yield v
+
+
+def summary_line(full):
+    """The bench line: the headline whole, every other leg as its figures.  It
+    stays below 2900 characters, short enough for a log that keeps the last
+    3000 (with the served sweeps it came to 22 000); --full prints all."""
+    top = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+           "vs_baseline", "dtype", "data")
+    out = {k: full[k] for k in top}
+    out["config"] = {k: full["config"][k] for k in ("workload", "log_n", "blowup_bits", "n_queries", "parallelism",
+                                                    "in_flight", "l2")}
+    out["config"]["in_flight"] = out["config"]["in_flight"].split(" (")[0]
+    out["e2e"] = {**full["e2e"], "api": full["e2e"]["api"].split(" ")[0]}
+    out["gpu_launches"] = full["gpu_launches"]
+    out["clocks"] = full["clocks"]
+    for k in ("value_one_in_flight", "p50_ms", "p99_ms", "lde_hbm_gbs"):
+        out[k] = full[k]
+    out["roofline"] = {k: full["roofline"][k] for k in ("bound", "achieved", "peak", "unit", "frac",
+                                                        "frac_of_nominal", "traffic")}
+    out["roofline"]["kernel"] = full["roofline"]["kernel"].split(":")[0]
+    out["lde_roofline"] = {k: full["lde_roofline"][k] for k in ("bound", "peak", "frac", "traffic")}
+    out["stages_ms"] = {k: float(f"{v:.4g}") for k, v in full["stages_ms"].items()}
+    kernels = {}  # [ms, share of its bound]
+    for leg in ("ntt_microbench", "kernel_microbench"):
+        for path, v in _timed_leaves(full.get(leg, {})):
+            if any("reference" in p for p in path):
+                continue
+            name = "/".join(p for p in path if p not in ("vortex", "evaluate", "interpolate"))
+            name = name.replace("_vortex", "")
+            if leg == "ntt_microbench":
+                name = "ntt_" + name + {"evaluate": "_e", "interpolate": "_i"}.get(path[-1], "")
+            frac = v.get("frac", v.get("frac_of_probe"))
+            kernels[name] = [float(f"{v['ms']:.4g}")] + ([round(frac, 3)] if frac is not None else [])
+    if kernels:
+        out["kernels"] = kernels
+    if "pow_grind" in full:
+        out["pow_grind"] = {k: full["pow_grind"][k] for k in ("candidates_per_s", "frac_of_probe")}
+    if "batched_commit" in full:
+        b = full["batched_commit"]
+        out["batched_commit"] = {"value": b["value"], "one_in_flight": b["value_one_in_flight"],
+                                 "e2e": b["e2e"]["value"]}
+    if "served" in full:
+        sv = full["served"]
+        out["served"] = {"plain_capacity": sv["plain_capacity_per_s"],
+                         "engine_peak": max(r["proofs_per_s"] for r in sv["served_sweep"]),
+                         "ratio_at_equal_p99": list(sv["speedup_at_equal_p99"].values())}
+    flags = list(_flags(full))
+    if flags:
+        out["outputs_equal"] = f"{sum(flags)}/{len(flags)}"
+    if "cpu_baseline" in full:
+        out["cpu_baseline"] = full["cpu_baseline"]
+    return _rounded(out)
+
+
 def max_over_ranks(values, dist, device="cpu"):
     """Each value's maximum over the ranks (a replica job is as slow as its
     slowest GPU); the values themselves when there is one rank."""
@@ -1134,6 +1216,7 @@ def main():
     ap.add_argument("--no-batched", action="store_true", help="skip the batched lifted commitment")
     ap.add_argument("--no-micro", action="store_true", help="skip the NTT / iNTT microbench (2^20, 2^24, 2^28)")
     ap.add_argument("--no-tune", action="store_true", help="keep the built-in NTT plans and leaf-kernel shapes")
+    ap.add_argument("--full", action="store_true", help="print every leg's whole object, sweeps and sources included")
     ap.add_argument("--kernels-only", action="store_true",
                     help="run only the standalone kernel microbench (Merkle, FRI folds, bit reversals) and print it")
     ap.add_argument("--kernel-log", type=int, default=26, help="log2 size of the standalone kernel microbench")
@@ -1436,7 +1519,7 @@ def main():
             cb = cpu_baseline(log_n)
             cb.pop("seconds", None)
             line["cpu_baseline"] = cb
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line) if args.full else json.dumps(summary_line(line), separators=(",", ":")), flush=True)
     cache.close()
     if dist is not None:
         dist.destroy_process_group()
