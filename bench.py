@@ -1111,7 +1111,7 @@ def summary_line(full):
     kernels = {}  # [ms, share of its bound]
     for leg in ("ntt_microbench", "kernel_microbench"):
         for path, v in _timed_leaves(full.get(leg, {})):
-            if any("reference" in p for p in path):
+            if any("reference" in p or "cpu" in p for p in path):
                 continue
             name = "/".join(p for p in path if p not in ("vortex", "evaluate", "interpolate"))
             name = name.replace("_vortex", "")

@@ -15,6 +15,9 @@
 // block runs: every block arrives at the cluster barrier first of all and
 // waits for the others right before its first remote store, so the wait is
 // over by then and costs nothing on the chain.
+//
+// Line folds of a log_n 10 proof: 88 us with a launch per layer, 82 with the
+// layers of at most 256 values in one block, 79-80 with the cluster above.
 #include <cooperative_groups.h>
 
 #include "vx_common.cuh"

@@ -364,13 +364,13 @@ __device__ __forceinline__ uint32_t chan_commit_quad(const Quad &q, const ChanSt
 //
 // Build: trees of depth <= 16 go to one multi-block reduce launch straight
 // from the leaves.  Deeper trees: one thread per 2^k-leaf subtree (k = 1..4,
-// tree_leaf_k), then node kernels of at most
-// 16 -> 1 down to 2^16 hashes, then the reduce launch for the rest.
-// The reduce kernel works in stages of up to 8 levels: each block reduces 256
-// hashes in shared memory, one compression per thread per level; the last
-// block of every group of 256 (found with a counter, no waiting) carries on
-// with the group's roots, and the block that reaches the root performs the
-// transcript step of the commitment.
+// tree_leaf_k), then node kernels of at most 16 -> 1 down to 2^16 hashes, then
+// the reduce launch for the rest.  The reduce kernel works in stages of up to
+// 8 levels: each block reduces 256 hashes in shared memory, a node per thread
+// at 128 nodes and per four lanes from 64 down; the last block of every group
+// of 256 (found with a counter, no waiting) carries on with the group's roots,
+// and the block that reaches the root performs the transcript step of the
+// commitment.
 struct TreeLevels {
     uint32_t n;            // number of stored levels including the leaf level
     uint32_t top;          // stored level the reduce kernel starts from (0: leaves)

@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(NT, min_blocks_for(NT)) ntt_tile_kernel(Pass2A
 }
 
 // Resident blocks per SM the vector pass is compiled for: 8 (64 registers)
-// against 6 or 5: 2^26 evaluate 381 us, 405 and 405; LDE of the 34-column
-// commitment 358 us against 384 with 6.
+// against 7, 6 and 5: 2^26 evaluate, one box, 389 us, 396, 405 and 405; LDE of the
+// 34-column commitment 358 us against 384 with 6.
 #ifndef VX_NTT_VEC_BLOCKS
 #define VX_NTT_VEC_BLOCKS 8
 #endif
@@ -399,9 +399,9 @@ __global__ void __launch_bounds__(NT, min_blocks_for(NT)) ntt_tile_kernel(Pass2A
 //  - Twiddles come from global memory as aligned runs of 1..16 words per
 //    layer; nothing is staged or decoded per tile.
 // Against 16 elements per thread with the tile and its twiddles staged in
-// shared memory (12.2-15.2 instructions per butterfly): 2^24 evaluate 134 ->
-// 108 us, interpolate 135 -> 120, 2^26 494 -> 381 and 504 -> 436, 16 columns
-// of 2^20 158 -> 101, each through its synchronous launcher.
+// shared memory (12.2-15.2 instructions per butterfly): 2^24 evaluate 130 ->
+// 106 us, interpolate 133 -> 111, 2^26 491 -> 385 and 501 -> 406, 16 columns
+// of 2^20 155 -> 96, each through its synchronous launcher.
 // A bottom pass (WL = 0, layers 0 .. R-1, R = 5..12) takes 4096 consecutive
 // elements, 2^(12-R) tiles, per block; an upper pass (R = 3..9, WL = 12 - R)
 // one tile of 2^R rows of 2^WL words.

@@ -7,10 +7,11 @@
 // v0' = v0 + v1, v1' = (v0 - v1) t, then scales by 2^-k (circle_ntt.cu:248-312).
 //
 // A pass applies the layers of one bit range [s, s + r) to tiles of
-// 2^r rows x 2^w columns held in shared memory; every element of a tile has
-// the same bits outside [s, s + r) except the w low column bits, so each
-// global row segment is 2^w contiguous words (w = min(s, 3) keeps segments at
-// one 32-byte sector).  A transform of 2^k points runs in ceil(k / 11) passes.
+// 2^r rows x 2^w columns; every element of a tile has the same bits outside
+// [s, s + r) except the w low column bits, so each global row segment is 2^w
+// contiguous words.  The passes of a transform are ntt_plan's: a bottom pass
+// (s = 0, w = 0) of up to 11 layers without tuning, then upper passes of 3 to
+// 8 layers on tiles of 2^12 elements (w = 12 - r).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

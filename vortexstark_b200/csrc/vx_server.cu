@@ -62,7 +62,8 @@ constexpr uint32_t kLargeLogEval = 24;
 constexpr uint32_t kMaxLargeInflight = 1;
 constexpr int kPrioDefault = 0;
 // A split large proof's tail: the line folds of layers of at most 2^16 values
-// (one latency-bound reduce launch each), queries and decommitment.
+// (a latency-bound launch each, one for those of at most 2^kTailLog together),
+// queries and decommitment.
 constexpr uint32_t kTailStage = 6;
 
 struct Slot {
