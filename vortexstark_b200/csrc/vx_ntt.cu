@@ -122,14 +122,15 @@ struct Pass2Args {
     uint32_t scale;   // output scale (1 = none)
     uint32_t vec;     // 1: columns and source 16-byte aligned, 4 consecutive elements per access
     uint32_t hb_log;  // > 0: the 2^hb_log tiles that read the same source tile are consecutive blocks
+    uint32_t tal;     // vector pass; 1: its twiddle runs allow load_run's wide loads (tables_aligned)
 };
-// What the vector pass needs beside it.  The 16-element pass is launched with
-// the above alone: 216 bytes of parameters; with these 232 a transform of
-// 2^11 to 2^19 elements took 0.3-0.5 us longer (2^14: 17.1 against 17.6 us).
+// What else the vector pass needs.  Apart because a launch with more than 224
+// bytes of parameters takes 0.3-0.5 us longer: with 232 the 16-element pass at
+// 2^14 17.6 us instead of 17.1, the vector pass at 2^22 38.1 instead of 37.5.
 struct VecArgs : Pass2Args {
-    uint64_t n_elems; // words per column
-    uint32_t tal;     // 1: the pass's twiddle runs allow load_run's wide loads (tables_aligned)
+    uint64_t n_elems;  // words per column
 };
+static_assert(sizeof(Pass2Args) == 216 && sizeof(VecArgs) == 224, "launch parameters");
 
 // Butterfly products: with a doubled twiddle (mmul_t2: one multiply, one
 // shift-add, one conditional subtract) or the plain one (mmul: a fold of the
