@@ -574,7 +574,7 @@ __device__ __forceinline__ uint32_t vec_base(uint32_t tid) {
 
 // PRE: every stage's twiddles are loaded along with the data, so their latencies
 // overlap; for launches of at most four blocks per SM, where nothing else
-// hides them and registers are free (launch_pass).
+// hides them and registers are free (figures at launch_pass).
 template <bool FWD, int R, int WL, int K>
 __device__ __forceinline__ void vec_prefetch(VecTw *tw, const VecArgs &p, const VecCtx &c) {
     using St = VecStage<FWD, R, WL, K>;
@@ -818,27 +818,26 @@ uint32_t sm_count() {
 }
 
 // The vector pass, or the 16-element one where a launch is too short for it:
-// from 2^11 (inverse: 2^10) to below 2^20 elements the chip is not full either
-// way, and twice the threads with half the work each finish first.  Launcher
-// times, 16-element against vector pass, us: 2^13 18.1 / 18.0 forward, 18.4 /
-// 18.8 inverse; 2^16 19.2 / 19.7 and 19.3 / 20.1; 2^19 20.6 / 21.3 and 20.5 /
-// 21.8; at the ends 2^10 15.1 / 15.3 and 15.3 / 15.8, 2^20 25.2 / 24.9 and
-// 25.1 / 25.2, 2^22 43.6 / 38.0 and 44.2 / 39.6 (runs of one side within 0.3).
-// Columns behind a device pointer array stay with the vector pass, whose
-// accesses are 16 bytes wide there too (16 x 2^16: 27.0 / 24.8).
-// PRE, with against without: forward 2^20 24.6 / 24.9, 3 x 2^18 22.2 / 22.6;
-// inverse 2^20 25.5 / 25.2, 8 x 2^16 23.4 / 23.0, but columns of one short
-// block 20 x 2^10 20.3 / 20.7, 2 x 2^10 17.2 / 17.7.
+// from 2^11 to below 2^20 elements the chip is not full either way, and twice
+// the threads with half the work each finish first.  Launcher times, 16-element
+// against vector pass, us: 2^13 18.1 / 18.0 forward, 18.4 / 18.8 inverse; 2^16
+// 19.2 / 19.7 and 19.3 / 20.1; 2^19 20.6 / 21.3 and 20.5 / 21.8; at the ends
+// 2^10 15.0 / 14.7 and 15.0 / 15.0, 2^20 25.2 / 24.6 and 25.2 / 25.1, 2^22 43.9 /
+// 37.8 and 44.4 / 39.2 (runs of one side within 0.3).  Columns behind a device
+// pointer array stay with the vector pass, whose accesses are 16 bytes wide
+// there too (8 x 2^14 22.2 / 21.4 and 22.1 / 21.7, 16 x 2^16 27.1 / 24.3).
+// PRE, with against without: 2^20 forward 24.6 / 24.9, 3 x 2^18 22.2 / 22.6; in
+// columns of 2^10 20 of them 19.9 / 20.7 inverse; longer inverse launches are
+// within 0.4 the other way (2^20 25.1 / 24.9, 8 x 2^16 23.1 / 22.7).
 template <bool FWD, int R, int WL>
 cudaError_t launch_pass(const VecArgs &a, uint64_t tiles, uint32_t n_cols, cudaStream_t st) {
     const uint64_t total = a.n_elems * n_cols;
-    if (!a.dev_cols && total >= (FWD ? 1ull << 11 : 1ull << 10) && total < (1ull << 20))
+    if (!a.dev_cols && total >= (1ull << 11) && total < (1ull << 20))
         return launch_pass2<FWD, R, WL>(a, tiles, n_cols, st);
     const uint64_t blocks = (a.n_elems + kVecTile - 1) / kVecTile;
     const dim3 grid((unsigned)blocks, n_cols);
-    if constexpr (FWD || (WL == 0 && R <= 10))
-        if ((FWD || a.n_elems <= 1024u) && blocks * n_cols <= sm_count() * kVecPreBlocks)
-            return launch_pdl(ntt_vec_kernel<FWD, R, WL, true>, grid, dim3(kVecThreads), 0, st, a);
+    if (blocks * n_cols <= sm_count() * kVecPreBlocks)
+        return launch_pdl(ntt_vec_kernel<FWD, R, WL, true>, grid, dim3(kVecThreads), 0, st, a);
     return launch_pdl(ntt_vec_kernel<FWD, R, WL, false>, grid, dim3(kVecThreads), 0, st, a);
 }
 
