@@ -47,6 +47,22 @@ def test_twiddle_tables(oracle, kind, k):
     assert np.array_equal(to_host(il, (1 << k) - 2), oil[:(1 << k) - 2])
 
 
+@pytest.mark.parametrize("left", [0x7FFFFFFF, 0xFFFFFFFF, 0x80000000, 0, 1])
+@pytest.mark.parametrize("k", [2, 4, 5, 7, 12])
+def test_twiddle_tables_in_used_memory(oracle, monkeypatch, k, left):
+    """Whatever the tables' memory held before."""
+    import torch
+
+    from vortexstark_b200 import circle
+    word = left - (1 << 32) if left >> 31 else left
+    monkeypatch.setattr(circle, "_u32", lambda n: torch.full((max(int(n), 1),), word, dtype=torch.int32, device="cuda"))
+    pc, oc = _cos(oracle, "half_coset", k)
+    il, ic, _, _ = circle.compute_inverse_twiddles_gpu(pc)
+    oil, oic, _ = oracle.twiddles(oc, True)
+    assert np.array_equal(to_host(ic, 1 << (k - 1)), oic)
+    assert np.array_equal(to_host(il, (1 << k) - 2), oil[:(1 << k) - 2])
+
+
 @pytest.mark.parametrize("kind", ["half_coset", "half_odds", "subgroup"])
 @pytest.mark.parametrize("k", [1, 2, 4, 7, 11, 12, 13, 16, 20])
 def test_ntt_evaluate_interpolate(oracle, kind, k):

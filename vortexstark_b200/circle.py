@@ -115,13 +115,15 @@ def compute_forward_twiddles_gpu(coset: Coset):
 
 
 def compute_inverse_twiddles_gpu(coset: Coset):
-    """circle.rs:525-550 — forward tables, then batch inverse (0 -> 0)."""
+    """circle.rs:525-550 — forward tables, then batch inverse (0 -> 0).  The
+    line table's last slot belongs to no layer and is never written: it stays
+    out of the inversion, whose chunks of 64 words share their products."""
     L = _lib.lib()
     line, circle, offsets, sizes = compute_forward_twiddles_gpu(coset)
     n = coset.size()
     iline, icircle = _u32(n - 1), _u32(n // 2)
-    if n - 1 > 0:
-        L.cuda_batch_inverse_m31(line.data_ptr(), iline.data_ptr(), n - 1)
+    if sum(sizes) > 0:
+        L.cuda_batch_inverse_m31(line.data_ptr(), iline.data_ptr(), sum(sizes))
     if n // 2 > 0:
         L.cuda_batch_inverse_m31(circle.data_ptr(), icircle.data_ptr(), n // 2)
     return iline, icircle, offsets, sizes
